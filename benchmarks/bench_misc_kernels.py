@@ -325,7 +325,7 @@ def case_latent(small):
                 keys = sum(min(i + 1, wd or n) for i in range(n)) * B
                 sec = timeit(lambda: ops.mla_prefill_attention(q, kv, got[:, C:], starts, klens, qsl, True, 0.07, n, out=out,
                                                                window=wd, sinks=s, want_lse=False))
-                report(f"prefill_umma_kernel (latent, {name})", sec, T * H * 256 * 2,
+                report(f"prefill_pair_kernel (latent, {name})", sec, T * H * 256 * 2,
                        f"{tag}; {keys * H * 640 / sec / 1e12:.0f} TFLOP/s of visible scores")
         else:
             sec = timeit(lambda: ops.absorb_query(q, w_uk, tab, C, C + R))

@@ -1,4 +1,4 @@
-"""MLA prefill: the up-projected 192 / 128 form on tcgen05 (csrc/attention/prefill_umma.cu, MLA instantiation; the
+"""MLA prefill: the up-projected 192 / 128 form on tcgen05 (csrc/attention/prefill_pair.cu, MLA instantiation; the
 kv_b_proj up-projection of the keys included) against the absorbed 576 / 512 form (the two per-head products around
 it included).  CUDA events, 3 warm-ups, median of 10; a 256 MB buffer is written between iterations (L2 flush).
 

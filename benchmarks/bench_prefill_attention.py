@@ -1,4 +1,4 @@
-"""Paged GQA prefill attention: the tcgen05 kernel (csrc/attention/prefill_umma.cu) against the mma.sync kernel
+"""Paged GQA prefill attention: the tcgen05 kernel (csrc/attention/prefill_pair.cu) against the mma.sync kernel
 (csrc/attention/paged_attention.cu).  CUDA events, 3 warm-ups, median of 10; a 256 MB buffer is written between
 iterations (L2 flush).
 
@@ -23,7 +23,6 @@ ap.add_argument("--q-len", type=int, default=2048)
 ap.add_argument("--ctx", type=int, default=0, help="cached tokens in front of the chunk")
 ap.add_argument("--heads", type=int, default=32)
 ap.add_argument("--kv-heads", type=int, default=8)
-ap.add_argument("--trace", action="store_true", help="phase timestamps of the tcgen05 kernel (one launch)")
 ap.add_argument("--bf16-tflops", type=float, default=1590.0, help="measured cuBLAS bf16 burst peak")
 a = ap.parse_args()
 dev, dt, D, bs = "cuda", torch.bfloat16, 128, 64
@@ -54,35 +53,12 @@ def timeit(fn):
     return statistics.median(ts)
 
 
-if a.trace:
-    from vllm_kunlun_b200.ops import _ext
-    C = _ext.C()
-    n_cta = B * a.heads * -(-QL // 128)
-    tr = torch.zeros(n_cta * 24, dtype=torch.int64, device=dev)
-    for _ in range(2):
-        tr.zero_()
-        C.set_kernel_trace(tr)
-        attention_cuda.paged_attention_cuda(out, q, cache, bt, sl, qsl, D ** -0.5, QL, S)
-        torch.cuda.synchronize()
-        C.set_kernel_trace(None)
-    t = tr.view(-1, 24).cpu()
-    t = t[(t[:, 0] > 0) & (t[:, 8] > 0)]
-    names = ["start", "first S", "t4 S seen", "t4 max done", "t4 P buffer free", "t4 P written", "loop done", "t5 S seen",
-             "t20 S seen", "t4 P seen by issuer", "end", "t4 S in registers", "t3 P.V issued", "t5 S issued"]
-    rel = t - t[:, :1]
-    print(f"# phase trace over {t.shape[0]} CTAs with > 20 tiles: ns after the CTA's own start (min / median / max)")
-    for i, nm in enumerate(names):
-        col = rel[:, i][t[:, i] > 0]
-        if col.numel():
-            print(f"{nm:>20}: {int(col.min()):8d} {int(col.median()):8d} {int(col.max()):8d}")
-    sys.exit(0)
-
 print(f"# prefill attention: {B} x {QL} query tokens over {S} keys, {a.heads} q / {a.kv_heads} kv heads, "
       f"{flops / 1e12:.3f} TFLOP (causal)")
 print("| kernel | ms | TFLOP/s | of measured bf16 peak |")
 print("|---|---|---|---|")
 res = {}
-for name, flag in (("tcgen05 (prefill_umma)", True), ("mma.sync (paged_attention)", False)):
+for name, flag in (("tcgen05 (prefill_pair)", True), ("mma.sync (paged_attention)", False)):
     attention_cuda.UMMA_PREFILL[0] = flag
     ms = timeit(lambda: attention_cuda.paged_attention_cuda(out, q, cache, bt, sl, qsl, D ** -0.5, QL, S))
     res[name] = out.float().clone()

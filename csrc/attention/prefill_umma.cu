@@ -1,4 +1,4 @@
-// Paged GQA prefill / chunked-prefill attention on tcgen05 + TMEM, fed by TMA straight from the paged KV cache
+// Paged GQA prefill / chunked-prefill attention with a score bias on tcgen05 + TMEM, fed by TMA straight from the paged KV cache
 // (head_dim 128, 16-bit).  The reference's `prefill_attention` call (v1/attention/backends/kunlun_attn.py:805-947).
 //
 // One CTA = (tile of 128 query rows of one request, one query head).  Per 128-key tile:
@@ -13,21 +13,16 @@
 // current one are issued as they become ready), warps 2-5 softmax + epilogue.  Two S buffers (2 x 128 TMEM columns)
 // + O (128 columns).  Causal masking by position (chunked prefill: row r of the request sits at ctx + r), optional
 // sliding window and attention sinks, optional log-sum-exp output.
-// `kBias`: a score bias per head and distance (query position minus key position) from a table [Hq][bias_len], whose last
-// entry serves every farther distance.  A tile that lies farther away altogether adds that constant inside the exponent; for
-// a nearer one the softmax warps put the 255 entries the tile can meet into shared memory (two buffers, one per tile parity).
-// `kSigmoid` (with `kBias`): a visible key counts with sigmoid(score + bias), not normalised - no maximum, no row sum and no
+// This kernel serves the forms with a score bias per head and distance (query position minus key position): a table [Hq]
+// [bias_len], whose last entry serves every farther distance (the forms without one run on prefill_pair.cu).  A tile that
+// lies farther away altogether adds that constant inside the exponent; for a nearer one the softmax warps put the 255 entries
+// the tile can meet into shared memory (two buffers, one per tile parity).
+// `kSigmoid`: a visible key counts with sigmoid(score + bias), not normalised - no maximum, no row sum and no
 // rescale; P.V accumulates as it is.  Rows need no statistics, so eight warps share the tile, two per 32 rows with half of the
 // keys (and, at the end, of the output dims) each.
-// `kKeep` (with `kBias`): with a window, the first keys of a request stay visible.  Their tiles come first in the tile list, which then
+// `kKeep`: with a window, the first keys of a request stay visible.  Their tiles come first in the tile list, which then
 // jumps to the window's first tile.
-// The MLA instantiation (`kMla`) is the compute-friendly prefill form of multi-head latent attention
-// (v1/attention/backends/mla/common.py:1782-1843): 192-dim q / k (128 "nope" dims per head + 64 rotary dims shared
-// by all heads), 128-dim v, keys and values read as contiguous rows of the up-projected `kv_b_proj` output
-// ([rows, heads * 256], k_nope | v per head) plus the rotary key rows ([rows, 64]); each request's keys start at
-// `kv_starts[req]`.  Causal (new tokens, possibly behind cached ones in front of the same rows; window and sinks as
-// above) or not (a chunk of cached context); the log-sum-exp output lets the caller merge chunks.  Its K ring has two 48 KB stages and V a single 32 KB one (208 KB of shared memory in all).
-// In both forms every head's output may be multiplied by sigmoid(gate[token, head]).
+// Every head's output may be multiplied by sigmoid(gate[token, head]).
 // TMA loads carry no cluster multicast.  Every wait is bounded; on time-out the status word is set and the CTA unwinds.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -47,14 +42,8 @@ constexpr int threads(bool sigmoid) { return 64 + 32 * soft_warps(sigmoid); }
 constexpr int kQTile = 128, kKTile = 128, kPage = 64, kD = 128;
 constexpr int kHalfBytes = 128 * 128;          // one 64-dim block of a 128-row operand tile
 constexpr int kOpBytes = 2 * kHalfBytes;       // Q, K, V or P tile: 32 KB
-constexpr int kStages = 2;                     // K ring
-template <bool kMla> struct Cfg {
-  static constexpr int kQBlocks = kMla ? 3 : 2;                 // 64-dim blocks of q / k
-  static constexpr int kKBytes = kQBlocks * kHalfBytes;         // Q tile or one K stage
-  static constexpr int kVStages = kMla ? 1 : 2;
-  static constexpr size_t kSmem = 1024 + (size_t)kStages * kKBytes + (size_t)kVStages * kOpBytes + kKBytes + kOpBytes + 256;
-  static constexpr size_t kBiasSmem = 2 * 256 * sizeof(float);
-};
+constexpr int kStages = 2;                     // K and V rings
+constexpr size_t kSmem = 1024 + (2 * kStages + 2) * (size_t)kOpBytes + 256 + 2 * 256 * sizeof(float);
 constexpr int kTmemCols = 512;                 // 2 x 128 (S) + 128 (O)
 constexpr float kMaxSlack = 8.f;
 
@@ -64,14 +53,12 @@ struct Params {
   const int* block_tables;  // [B, max_blocks]
   const int* seq_lens;
   const int* qsl;
-  const int* kv_starts;     // MLA form: first key row of each request in the contiguous K / V tensors
   const float* sinks;       // [Hq] or null
-  const float* bias;        // [Hq][bias_len] score bias by distance (kBias)
+  const float* bias;        // [Hq][bias_len] score bias by distance
   const void* gate;         // [T, >= Hq] in the output's type, or null
   int64_t gate_stride;
   int* status;
-  unsigned long long* trace;   // optional phase timestamps [CTA][24] (null = off)
-  int Hq, Hkv, block_size, max_blocks, window, keep_first, causal, bias_len;
+  int Hq, Hkv, block_size, max_blocks, window, keep_first, bias_len;
   int64_t num_blocks;
   float scale_log2;
 };
@@ -141,18 +128,16 @@ template <> __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) 
   return (uint32_t)__half_as_ushort(__float2half(a)) | ((uint32_t)__half_as_ushort(__float2half(b)) << 16);
 }
 
-template <typename T, bool kMla, bool kBias, bool kSigmoid, bool kKeep>
+template <typename T, bool kSigmoid, bool kKeep>
 __global__ void __launch_bounds__(threads(kSigmoid))
 prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKV,
-                    const __grid_constant__ CUtensorMap tmKpe, const __grid_constant__ Params p) {
-  static_assert(!kSigmoid || (kBias && !kMla));
+                    const __grid_constant__ Params p) {
   constexpr int kSoftWarps = soft_warps(kSigmoid);
-  constexpr int kQBlocks = Cfg<kMla>::kQBlocks, kKBytes = Cfg<kMla>::kKBytes, kVStages = Cfg<kMla>::kVStages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sVr = smem + kStages * kKBytes;          // V ring: [kVStages][2 dim blocks][128 keys][128 B]
-  uint8_t* sQ = sVr + kVStages * kOpBytes;          // [kQBlocks dim blocks][128 rows][128 B]
-  uint8_t* sP = sQ + kKBytes;                       // [2 key blocks][128 rows][128 B]
+  uint8_t* sVr = smem + kStages * kOpBytes;          // V ring: [kStages][2 dim blocks][128 keys][128 B]
+  uint8_t* sQ = sVr + kStages * kOpBytes;          // [2 dim blocks][128 rows][128 B]
+  uint8_t* sP = sQ + kOpBytes;                       // [2 key blocks][128 rows][128 B]
   uint64_t* bars = reinterpret_cast<uint64_t*>(sP + kOpBytes);
   uint64_t* q_full = bars;             // [1]
   uint64_t* k_full = bars + 1;         // [2]
@@ -163,16 +148,14 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint64_t* p_free = bars + 10;        // [1]
   uint64_t* o_done = bars + 11;        // [1] one phase per P.V
   uint64_t* o_final = bars + 12;       // [1] once, after the last P.V
-  uint64_t* v_full = bars + 13;        // [2] (kVStages used)
+  uint64_t* v_full = bars + 13;        // [2] (kStages used)
   uint64_t* v_empty = bars + 15;       // [2] P.V of the tile has been computed
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* sBias = reinterpret_cast<float*>(sP + kOpBytes + 256);   // [2][256] (kBias)
+  float* sBias = reinterpret_cast<float*>(sP + kOpBytes + 256);   // [2][256]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   Abort ab{p.status, abort_flag};
-  const int cta_id = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-  if (threadIdx.x == 64) trace_mark(p.trace, cta_id, 0);
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     mbar_init(q_full, 1);
@@ -185,7 +168,6 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     mbar_fence_init();
     prefetch_tmap(&tmQ);
     prefetch_tmap(&tmKV);
-    if (kMla) prefetch_tmap(&tmKpe);
     griddep_launch();
   }
   if (warp == 1) {
@@ -202,8 +184,7 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const int kvh = head / (p.Hq / p.Hkv);
   const int qs = p.qsl[req], q_len = p.qsl[req + 1] - qs;
   const int seq_len = p.seq_lens[req];
-  // not causal: every row sees all of the request's keys - as if it sat far behind them
-  const int ctx = (kMla && !p.causal) ? (1 << 29) : seq_len - q_len;
+  const int ctx = seq_len - q_len;
   const int row0 = blockIdx.x * kQTile;                      // first query row of this tile within the request
   const int n_rows = max(0, min(kQTile, q_len - row0));
   // keys visible to the tile: up to the position of its last row; with a window, from the first row's window start
@@ -220,12 +201,11 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (elect_one() && n_tiles > 0) {
-      mbar_expect_tx(q_full, kKBytes);
+      mbar_expect_tx(q_full, kOpBytes);
 #pragma unroll
-      for (int h = 0; h < kQBlocks; ++h)
-        tma_load_2d(sQ + h * kHalfBytes, &tmQ, q_full, head * (kQBlocks * 64) + h * 64, qs + row0);
-      const int* bt = kMla ? nullptr : p.block_tables + (int64_t)req * p.max_blocks;
-      const int kv_row0 = kMla ? p.kv_starts[req] : 0;
+      for (int h = 0; h < 2; ++h)
+        tma_load_2d(sQ + h * kHalfBytes, &tmQ, q_full, head * (kD) + h * 64, qs + row0);
+      const int* bt = p.block_tables + (int64_t)req * p.max_blocks;
       // cache row of a key's page (paged form): masked keys read any initialised page
       auto page_row = [&](int key) -> int64_t {
         const int bi = key / p.block_size;
@@ -236,43 +216,30 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       auto load_k = [&](int i) -> bool {
         const int stage = i & 1;
         if (i >= kStages && !wait_or_abort(&k_empty[stage], ((i >> 1) - 1) & 1, ab, 801)) return false;
-        mbar_expect_tx(&k_full[stage], kKBytes);
-        uint8_t* sK = smem + stage * kKBytes;
+        mbar_expect_tx(&k_full[stage], kOpBytes);
+        uint8_t* sK = smem + stage * kOpBytes;
 #pragma unroll
         for (int pg = 0; pg < kKTile / kPage; ++pg) {
           const int key = tile_key(i) + pg * kPage;
           uint8_t* dst = sK + pg * (kPage * 128);
-          if constexpr (kMla) {
-            // rows past the request's keys belong to the next request or lie outside the tensor (zero fill): masked
+          const int64_t rowK = page_row(key);
 #pragma unroll
-            for (int h = 0; h < 2; ++h) tma_load_2d(dst + h * kHalfBytes, &tmKV, &k_full[stage], head * 256 + h * 64, kv_row0 + key);
-            tma_load_2d(dst + 2 * kHalfBytes, &tmKpe, &k_full[stage], 0, kv_row0 + key);
-          } else {
-            const int64_t rowK = page_row(key);
-#pragma unroll
-            for (int h = 0; h < 2; ++h) tma_load_2d(dst + h * kHalfBytes, &tmKV, &k_full[stage], h * 64, (int)rowK);
-          }
+          for (int h = 0; h < 2; ++h) tma_load_2d(dst + h * kHalfBytes, &tmKV, &k_full[stage], h * 64, (int)rowK);
         }
         return true;
       };
       auto load_v = [&](int i) -> bool {
-        const int stage = i % kVStages, use = i / kVStages;
-        if (i >= kVStages && !wait_or_abort(&v_empty[stage], (use - 1) & 1, ab, 804)) return false;
+        const int stage = i % kStages, use = i / kStages;
+        if (i >= kStages && !wait_or_abort(&v_empty[stage], (use - 1) & 1, ab, 804)) return false;
         mbar_expect_tx(&v_full[stage], kOpBytes);
         uint8_t* sV = sVr + stage * kOpBytes;
 #pragma unroll
         for (int pg = 0; pg < kKTile / kPage; ++pg) {
           const int key = tile_key(i) + pg * kPage;
           uint8_t* dst = sV + pg * (kPage * 128);
-          if constexpr (kMla) {
+          const int64_t rowV = page_row(key) + (int64_t)p.Hkv * p.block_size;
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
-              tma_load_2d(dst + h * kHalfBytes, &tmKV, &v_full[stage], head * 256 + 128 + h * 64, kv_row0 + key);
-          } else {
-            const int64_t rowV = page_row(key) + (int64_t)p.Hkv * p.block_size;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) tma_load_2d(dst + h * kHalfBytes, &tmKV, &v_full[stage], h * 64, (int)rowV);
-          }
+          for (int h = 0; h < 2; ++h) tma_load_2d(dst + h * kHalfBytes, &tmKV, &v_full[stage], h * 64, (int)rowV);
         }
         return true;
       };
@@ -293,9 +260,9 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         for (int i = max(0, issued_k - kStages); i < issued_k; ++i)
           for (uint32_t q2 = 0; q2 < (1u << 16); ++q2)
             if (mbar_try_wait(&k_full[i & 1], (i >> 1) & 1)) break;
-        for (int i = max(0, issued_v - kVStages); i < issued_v; ++i)
+        for (int i = max(0, issued_v - kStages); i < issued_v; ++i)
           for (uint32_t q2 = 0; q2 < (1u << 16); ++q2)
-            if (mbar_try_wait(&v_full[i % kVStages], (i / kVStages) & 1)) break;
+            if (mbar_try_wait(&v_full[i % kStages], (i / kStages) & 1)) break;
       }
     }
   } else if (warp == 1) {
@@ -308,29 +275,27 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       const uint32_t q_addr = smem_u32(sQ), p_addr = smem_u32(sP);
       auto issue_s = [&](int i) {
         tc_fence_after_sync();
-        const uint32_t k_addr = smem_u32(smem + (i & 1) * kKBytes);
+        const uint32_t k_addr = smem_u32(smem + (i & 1) * kOpBytes);
 #pragma unroll
-        for (int k = 0; k < kQBlocks * 4; ++k) {
+        for (int k = 0; k < kD / 16; ++k) {
           const int kb = k / 4, kk = k % 4;
           umma_f16(tS + (i & 1) * kKTile, umma_desc_k_sw128(q_addr + kb * kHalfBytes + kk * 32),
                    umma_desc_k_sw128(k_addr + kb * kHalfBytes + kk * 32), idesc_s, k > 0 ? 1u : 0u);
         }
         umma_commit(&s_full[i & 1]);
         umma_commit(&k_empty[i & 1]);
-        if (i == 5) trace_mark(p.trace, cta_id, 13);
       };
       auto issue_pv = [&](int i) {
         tc_fence_after_sync();
-        const uint32_t v_addr = smem_u32(sVr + (i % kVStages) * kOpBytes);
+        const uint32_t v_addr = smem_u32(sVr + (i % kStages) * kOpBytes);
 #pragma unroll
         for (int k = 0; k < kKTile / 16; ++k) {
           // A: 16 keys of P (key block k / 4, 32 bytes in); B: the same 16 keys of V, 128 dims (two 64-dim blocks)
           umma_f16(tO, umma_desc_k_sw128(p_addr + (k / 4) * kHalfBytes + (k % 4) * 32),
                    umma_desc_mn_sw128(v_addr + k * 2048, kHalfBytes, 1024), idesc_o, (i > 0 || k > 0) ? 1u : 0u);
         }
-        if (i == 3) trace_mark(p.trace, cta_id, 12);
         umma_commit(o_done);   // first: whoever has seen p_free of this tile may rely on o_done having advanced
-        umma_commit(&v_empty[i % kVStages]);
+        umma_commit(&v_empty[i % kStages]);
         umma_commit(p_free);
         if (i == n_tiles - 1) umma_commit(o_final);
       };
@@ -346,8 +311,7 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           progressed = true;
         }
         if (next_pv < next_s && mbar_try_wait(p_ready, next_pv & 1) &&
-            mbar_try_wait(&v_full[next_pv % kVStages], (next_pv / kVStages) & 1)) {
-          if (next_pv == 4) trace_mark(p.trace, cta_id, 9);
+            mbar_try_wait(&v_full[next_pv % kStages], (next_pv / kStages) & 1)) {
           issue_pv(next_pv);
           ++next_pv;
           progressed = true;
@@ -370,30 +334,24 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     float m_used = -INFINITY, l_sum = 0.f;
     bool fail = false;
     constexpr float kLog2e = 1.4426950408889634f;
-    const float* bias = kBias ? p.bias + (int64_t)head * p.bias_len : nullptr;
-    const float far_bias = kBias ? bias[p.bias_len - 1] * kLog2e : 0.f;
+    const float* bias = p.bias + (int64_t)head * p.bias_len;
+    const float far_bias = bias[p.bias_len - 1] * kLog2e;
     for (int i = 0; i < n_tiles; ++i) {
       const int buf = i & 1;
       if (!fail && !wait_or_abort(&s_full[buf], (i >> 1) & 1, ab, 805)) fail = true;
       tc_fence_after_sync();
-      if (threadIdx.x == 64 && i == 0) trace_mark(p.trace, cta_id, 1);
-      if (threadIdx.x == 64 && i == 4) trace_mark(p.trace, cta_id, 2);
-      if (threadIdx.x == 64 && i == 5) trace_mark(p.trace, cta_id, 7);
-      if (threadIdx.x == 64 && i == 20) trace_mark(p.trace, cta_id, 8);
       const int key0 = tile_key(i);
       const bool full_tile = key0 + kKTile - 1 <= pos_first && key0 + kKTile <= kv_end &&
                              (p.window <= 0 || key0 > pos_last - p.window || (kKeep && key0 + kKTile <= kept));
       // nearest distance of the tile: beyond the table's last entry its bias is one constant
-      const bool near_tile = kBias && p.bias_len > 1 && pos_first - (key0 + kKTile - 1) < p.bias_len - 1;
-      if constexpr (kBias) {
-        if (near_tile) {   // entry d: distance pos_first - key0 - 127 + d
-          float* dst = sBias + (i & 1) * 256;
-          const int tid = threadIdx.x - 64, d0 = pos_first - key0 - (kKTile - 1);
+      const bool near_tile = p.bias_len > 1 && pos_first - (key0 + kKTile - 1) < p.bias_len - 1;
+      if (near_tile) {   // entry d: distance pos_first - key0 - 127 + d
+        float* dst = sBias + (i & 1) * 256;
+        const int tid = threadIdx.x - 64, d0 = pos_first - key0 - (kKTile - 1);
 #pragma unroll
-          for (int d = 0; d < 256; d += 32 * kSoftWarps)
-            dst[tid + d] = bias[min(max(d0 + tid + d, 0), p.bias_len - 1)] * kLog2e;
-          asm volatile("bar.sync 3, %0;" ::"n"(32 * kSoftWarps) : "memory");
-        }
+        for (int d = 0; d < 256; d += 32 * kSoftWarps)
+          dst[tid + d] = bias[min(max(d0 + tid + d, 0), p.bias_len - 1)] * kLog2e;
+        asm volatile("bar.sync 3, %0;" ::"n"(32 * kSoftWarps) : "memory");
       }
       // ---- the whole row (128 scores) in one TMEM round trip: a tcgen05.ld + wait pair costs several hundred
       // nanoseconds whatever its width, so all four 32-column loads are issued before the single wait, and the
@@ -402,7 +360,6 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #pragma unroll
       for (int c = 0; c < kCols; c += 32) tmem_ld_x32_p(tS + buf * kKTile + col0 + c, v + c);
       tmem_ld_wait();
-      if (threadIdx.x == 64 && i == 4) trace_mark(p.trace, cta_id, 11);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&s_empty[buf]);
@@ -410,14 +367,12 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       // row maximum runs on four partial maxima and the exponentials in chunks of 32 with four partial sums; the
       // raw scores are masked in place and scaled inside the exponent (one FMA + one ex2 per element).
       float sc = p.scale_log2, off = far_bias;     // exponent = raw score * sc + off - maximum
-      if constexpr (kBias) {
-        if (near_tile) {
-          const float* src = sBias + (i & 1) * 256 + (kKTile - 1) + r - col0;
+      if (near_tile) {
+        const float* src = sBias + (i & 1) * 256 + (kKTile - 1) + r - col0;
 #pragma unroll
-          for (int e = 0; e < kCols; ++e) v[e] = __float_as_uint(fmaf(__uint_as_float(v[e]), p.scale_log2, src[-e]));
-          sc = 1.f;
-          off = 0.f;
-        }
+        for (int e = 0; e < kCols; ++e) v[e] = __float_as_uint(fmaf(__uint_as_float(v[e]), p.scale_log2, src[-e]));
+        sc = 1.f;
+        off = 0.f;
       }
       if (!full_tile) {
 #pragma unroll
@@ -466,9 +421,8 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         for (int u = 0; u < 4; ++u) mx[u] = fmaxf(mx[u], __uint_as_float(v[e + u]));
       }
       float tmax = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sc;   // scale > 0: max commutes
-      if (kBias) tmax += off;
+      tmax += off;
       if (!row_ok) tmax = -INFINITY;
-      if (threadIdx.x == 64 && i == 4) trace_mark(p.trace, cta_id, 3);
       // ---- lazy running maximum; the rescale of O is warp-collective (TMEM access), so the warp decides together
       float alpha = 1.f;
       const bool bump = tmax > m_used + kMaxSlack;
@@ -476,7 +430,6 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       // P (one buffer): the previous P.V must have read it (it has, long ago, unless the tensor pipe is behind);
       // this also keeps o_done within one phase
       if (i >= 1 && !fail && !wait_or_abort(p_free, (i - 1) & 1, ab, 806)) fail = true;
-      if (threadIdx.x == 64 && i == 4) trace_mark(p.trace, cta_id, 4);
       if (__any_sync(0xffffffffu, bump) && i > 0) {
         if (!fail && !wait_or_abort(o_done, (i - 1) & 1, ab, 808)) fail = true;
         tc_fence_after_sync();
@@ -494,7 +447,7 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       // ---- exponentials, row sum and the P row (16-bit, K-major over keys, 16-byte chunks swizzled by row; keys
       // 8 q .. 8 q + 7 = chunk q % 8 of key block q / 8), 32 keys at a time
       float neg_ms = (m_used == -INFINITY || !row_ok) ? -INFINITY : -m_used;   // invalid rows: P = 0
-      if (kBias) neg_ms += off;
+      neg_ms += off;
       float ls[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int c = 0; c < kKTile; c += 32) {
@@ -525,10 +478,8 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       const bool warp_failed = __any_sync(0xffffffffu, fail);
       __syncwarp();
       if (lane == 0 && !warp_failed) mbar_arrive(p_ready);
-      if (threadIdx.x == 64 && i == 4) trace_mark(p.trace, cta_id, 5);
       }
     }
-    if (threadIdx.x == 64) trace_mark(p.trace, cta_id, 6);
     // ---- epilogue
     bool ok = !fail;
     if (ok && n_tiles > 0) {
@@ -568,22 +519,20 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   tc_fence_before_sync();
   __syncthreads();
-  if (threadIdx.x == 64) trace_mark(p.trace, cta_id, 10);
   if (warp == 1) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, kTmemCols);
   }
 }
 
-template <typename T, bool kMla, bool kBias, bool kSigmoid, bool kKeep>
-static int launch(const Params& p, const CUtensorMap& tmQ, const CUtensorMap& tmKV, const CUtensorMap& tmKpe, int B,
+template <typename T, bool kSigmoid, bool kKeep>
+static int launch(const Params& p, const CUtensorMap& tmQ, const CUtensorMap& tmKV, int B,
                   int max_query_len, cudaStream_t st) {
-  auto kern = prefill_umma_kernel<T, kMla, kBias, kSigmoid, kKeep>;
-  const size_t smem = Cfg<kMla>::kSmem + (kBias ? Cfg<kMla>::kBiasSmem : 0);
-  cudaError_t e = ensure_dynamic_smem((const void*)kern, (int)smem);
+  auto kern = prefill_umma_kernel<T, kSigmoid, kKeep>;
+  cudaError_t e = ensure_dynamic_smem((const void*)kern, (int)kSmem);
   if (e != cudaSuccess) return (int)e;
   dim3 grid((unsigned)((max_query_len + kQTile - 1) / kQTile), (unsigned)p.Hq, (unsigned)B);
-  return (int)launch_pdl(kern, grid, dim3(threads(kSigmoid)), smem, st, tmQ, tmKV, tmKpe, p);
+  return (int)launch_pdl(kern, grid, dim3(threads(kSigmoid)), kSmem, st, tmQ, tmKV, p);
 }
 
 }  // namespace pattn
@@ -591,64 +540,33 @@ static int launch(const Params& p, const CUtensorMap& tmQ, const CUtensorMap& tm
 
 // Paged GQA prefill attention on tcgen05 (head_dim 128, block_size a multiple of 64).  `tmQ`: q as a 2-D
 // [T, Hq * 128] 16-bit tensor with 64-column x 128-row boxes; `tmKV`: the cache as [rows, 128] with 64 x 64 boxes;
-// both with 128-byte swizzle.  `bias` [Hq][bias_len] (or null): score bias by distance, the last entry for all farther ones;
-// `gate` [T][>= Hq] (or null): raw output gates; `sigmoid`: weights without a softmax (needs a bias; no sinks, no lse);
-// `keep_first`: keys that a window never hides (needs a bias).  Returns 3 for shapes it does not serve.
+// both with 128-byte swizzle.  `bias` [Hq][bias_len]: score bias by distance, the last entry for all farther ones;
+// `gate` [T][>= Hq] (or null): raw output gates; `sigmoid`: weights without a softmax (no sinks, no lse);
+// `keep_first`: keys that a window never hides.  Returns 3 for shapes it does not serve.
 extern "C" int b200_prefill_attention_umma(void* out, float* lse, const void* tmQ, const void* tmKV,
                                            const int* block_tables, const int* seq_lens, const int* qsl,
                                            const float* sinks, int* status, int B, int Hq, int Hkv, int D, int block_size,
                                            int max_blocks, int64_t num_blocks, int max_query_len, int window, float scale,
                                            const float* bias, int bias_len, const void* gate, int64_t gate_stride,
-                                           int keep_first, int sigmoid, int dtype, unsigned long long* trace,
-                                           cudaStream_t st) {
+                                           int keep_first, int sigmoid, int dtype, cudaStream_t st) {
   using namespace b200;
   if (B == 0 || max_query_len <= 0) return 0;
-  if ((bias != nullptr && bias_len < 1) || keep_first < 0) return 2;
-  if (keep_first > 0 && bias == nullptr) return 2;
-  if (sigmoid && (bias == nullptr || sinks != nullptr || lse != nullptr)) return 2;
+  if (bias == nullptr || bias_len < 1 || keep_first < 0) return 2;
+  if (sigmoid && (sinks != nullptr || lse != nullptr)) return 2;
   if (D != 128 || Hq % Hkv || block_size % pattn::kPage || B > 65535 || Hq > 65535) return 3;
   pattn::Params p;
   p.out = out; p.lse = lse; p.block_tables = block_tables; p.seq_lens = seq_lens; p.qsl = qsl; p.sinks = sinks;
-  p.status = status; p.trace = trace; p.Hq = Hq; p.Hkv = Hkv; p.block_size = block_size; p.max_blocks = max_blocks; p.window = window; p.keep_first = keep_first;
+  p.status = status; p.Hq = Hq; p.Hkv = Hkv; p.block_size = block_size; p.max_blocks = max_blocks; p.window = window; p.keep_first = keep_first;
   p.num_blocks = num_blocks; p.scale_log2 = scale * 1.4426950408889634f;
-  p.kv_starts = nullptr; p.causal = 1; p.gate = gate; p.gate_stride = gate_stride; p.bias = bias; p.bias_len = bias_len;
+  p.gate = gate; p.gate_stride = gate_stride; p.bias = bias; p.bias_len = bias_len;
   const CUtensorMap& q = *reinterpret_cast<const CUtensorMap*>(tmQ);
   const CUtensorMap& kv = *reinterpret_cast<const CUtensorMap*>(tmKV);
-#define B200_PA_LAUNCH(T)                                                                            \
-  (sigmoid           ? pattn::launch<T, false, true, true, true>(p, q, kv, kv, B, max_query_len, st)  \
-   : keep_first > 0  ? pattn::launch<T, false, true, false, true>(p, q, kv, kv, B, max_query_len, st) \
-   : bias != nullptr ? pattn::launch<T, false, true, false, false>(p, q, kv, kv, B, max_query_len, st) \
-                     : pattn::launch<T, false, false, false, false>(p, q, kv, kv, B, max_query_len, st))
+#define B200_PA_LAUNCH(T)                                                             \
+  (sigmoid          ? pattn::launch<T, true, true>(p, q, kv, B, max_query_len, st)    \
+   : keep_first > 0 ? pattn::launch<T, false, true>(p, q, kv, B, max_query_len, st)   \
+                    : pattn::launch<T, false, false>(p, q, kv, B, max_query_len, st))
   if (dtype == 1) return B200_PA_LAUNCH(__nv_bfloat16);
   if (dtype == 2) return B200_PA_LAUNCH(__half);
 #undef B200_PA_LAUNCH
-  return 3;
-}
-
-// Multi-head latent attention prefill in the compute-friendly form (192-dim q / k, 128-dim v) on tcgen05.
-// `tmQ`: q as [T, Hq * 192] with 64-column x 128-row boxes; `tmKV`: the up-projected keys / values as
-// [rows, Hq * 256] (k_nope | v per head) with 64 x 64 boxes; `tmKpe`: the rotary keys as [rows, 64] with 64 x 64
-// boxes; all 16-bit with 128-byte swizzle and row extents equal to the number of valid rows.  Request r owns key rows
-// kv_starts[r] .. kv_starts[r] + kv_lens[r] and query rows qsl[r] .. qsl[r + 1]; causal: its queries are its last
-// keys.  Rows of requests with no key are not written (the caller presets out = 0, lse = -inf).
-extern "C" int b200_mla_prefill_umma(void* out, float* lse, const void* tmQ, const void* tmKV, const void* tmKpe,
-                                     const int* kv_starts, const int* kv_lens, const int* qsl, const float* sinks,
-                                     const void* gate, int64_t gate_stride, int* status, int B, int Hq,
-                                     int max_query_len, int causal, int window, float scale, int dtype,
-                                     unsigned long long* trace, cudaStream_t st) {
-  using namespace b200;
-  if (B == 0 || max_query_len <= 0) return 0;
-  if (B > 65535 || Hq > 65535) return 3;
-  if (window < 0 || (window > 0 && !causal)) return 2;
-  pattn::Params p;
-  p.out = out; p.lse = lse; p.block_tables = nullptr; p.seq_lens = kv_lens; p.qsl = qsl; p.kv_starts = kv_starts;
-  p.sinks = sinks; p.bias = nullptr; p.bias_len = 0; p.gate = gate; p.gate_stride = gate_stride; p.status = status; p.trace = trace; p.Hq = Hq; p.Hkv = Hq; p.block_size = pattn::kPage;
-  p.max_blocks = 0; p.window = window; p.keep_first = 0; p.causal = causal ? 1 : 0; p.num_blocks = 0;
-  p.scale_log2 = scale * 1.4426950408889634f;
-  const CUtensorMap& q = *reinterpret_cast<const CUtensorMap*>(tmQ);
-  const CUtensorMap& kv = *reinterpret_cast<const CUtensorMap*>(tmKV);
-  const CUtensorMap& kpe = *reinterpret_cast<const CUtensorMap*>(tmKpe);
-  if (dtype == 1) return pattn::launch<__nv_bfloat16, true, false, false, false>(p, q, kv, kpe, B, max_query_len, st);
-  if (dtype == 2) return pattn::launch<__half, true, false, false, false>(p, q, kv, kpe, B, max_query_len, st);
   return 3;
 }

@@ -1002,7 +1002,6 @@ void decode_attention_umma(at::Tensor out, const at::Tensor& q, const at::Tensor
                                    early_meta ? 1 : 0, BIAS_GATE_ARGS, (int)keep_first, sigmoid, dtype_code(q), stream()), "decode_attention_umma");
 }
 
-extern at::Tensor g_kernel_trace;
 // Paged GQA prefill attention on tcgen05 (head_dim 128): q [T, Hq, 128], kv_cache [blocks, 2, Hkv, block_size, 128];
 // optional lse [T, Hq] (natural log).
 void prefill_attention_umma(at::Tensor out, const at::Tensor& q, const at::Tensor& kv_cache, const at::Tensor& block_tables,
@@ -1031,15 +1030,23 @@ void prefill_attention_umma(at::Tensor out, const at::Tensor& q, const at::Tenso
   at::Tensor flat = kv_cache.view({-1, 128});
   const Tmap& tq = get_tmap(gs, q2, 128, 2);
   const Tmap& tk = get_tmap(gs, flat, 64, 2);
+  if (!bias.has_value() && !sigmoid && keep_first == 0) {
+    check(b200_prefill_attention_pair(out.data_ptr(), lse.has_value() ? lse->data_ptr<float>() : nullptr, tq.b, tk.b,
+                                      block_tables.data_ptr<int>(), seq_lens.data_ptr<int>(), qsl.data_ptr<int>(),
+                                      sinks.has_value() ? sinks->data_ptr<float>() : nullptr, gs.status.data_ptr<int>(),
+                                      (int)seq_lens.size(0), (int)q.size(1), (int)kv_cache.size(2), 128,
+                                      (int)kv_cache.size(3), (int)block_tables.stride(0), kv_cache.size(0),
+                                      (int)max_query_len, (int)window, (float)scale, opt_ptr(gate),
+                                      gate.has_value() ? gate->stride(0) : 0, dtype_code(q), gs.num_sms, stream()),
+          "prefill_attention_pair");
+    return;
+  }
   check(b200_prefill_attention_umma(out.data_ptr(), lse.has_value() ? lse->data_ptr<float>() : nullptr, tq.b, tk.b,
                                     block_tables.data_ptr<int>(), seq_lens.data_ptr<int>(), qsl.data_ptr<int>(),
                                     sinks.has_value() ? sinks->data_ptr<float>() : nullptr, gs.status.data_ptr<int>(),
                                     (int)seq_lens.size(0), (int)q.size(1), (int)kv_cache.size(2), 128, (int)kv_cache.size(3),
                                     (int)block_tables.stride(0), kv_cache.size(0), (int)max_query_len, (int)window,
                                     (float)scale, BIAS_GATE_ARGS, (int)keep_first, sigmoid, dtype_code(q),
-                                    (g_kernel_trace.defined() &&
-                                     g_kernel_trace.numel() >= (int64_t)seq_lens.size(0) * q.size(1) * ((max_query_len + 127) / 128) * 24)
-                                        ? reinterpret_cast<unsigned long long*>(g_kernel_trace.data_ptr<int64_t>()) : nullptr,
                                     stream()),
         "prefill_attention_umma");
 }
@@ -1082,14 +1089,11 @@ void mla_prefill_umma(at::Tensor out, const at::Tensor& q, const at::Tensor& kv,
   const Tmap& tk = get_tmap(gs, kv, 64, 2);
   const Tmap& tp = get_tmap(gs, k_pe, 64, 2);
   const int B = (int)kv_lens.numel();
-  check(b200_mla_prefill_umma(out.data_ptr(), lse.has_value() ? lse->data_ptr<float>() : nullptr, tq.b, tk.b, tp.b,
+  check(b200_mla_prefill_pair(out.data_ptr(), lse.has_value() ? lse->data_ptr<float>() : nullptr, tq.b, tk.b, tp.b,
                               kv_starts.data_ptr<int>(), kv_lens.data_ptr<int>(), qsl.data_ptr<int>(),
                               sinks.has_value() ? sinks->data_ptr<float>() : nullptr, opt_ptr(gate),
                               gate.has_value() ? gate->stride(0) : 0, gs.status.data_ptr<int>(), B, (int)q.size(1),
-                              (int)max_query_len, causal ? 1 : 0, (int)window, (float)scale, dtype_code(q),
-                              (g_kernel_trace.defined() &&
-                               g_kernel_trace.numel() >= (int64_t)B * q.size(1) * ((max_query_len + 127) / 128) * 24)
-                                  ? reinterpret_cast<unsigned long long*>(g_kernel_trace.data_ptr<int64_t>()) : nullptr,
+                              (int)max_query_len, causal ? 1 : 0, (int)window, (float)scale, dtype_code(q), gs.num_sms,
                               stream()),
         "mla_prefill_umma");
 }

@@ -510,6 +510,31 @@ def test_prefill_attention_umma(Hq, Hkv, bs, dtype):
     torch.testing.assert_close(lse.cpu(), torch.stack(want), atol=2e-2, rtol=2e-3)
 
 
+@pytest.mark.parametrize("Hq,Hkv", [(12, 2), (6, 2), (5, 5)])
+@pytest.mark.parametrize("window", [0, 100, 128, 300])
+def test_prefill_attention_pairs(Hq, Hkv, window):
+    """Prefill attention with two query tiles per CTA - two heads (12 / 2) or two row tiles (6 / 2: three heads per key head, 5 /
+    5) - against the fp32 oracle: more work items than CTAs, tiles whose partner is empty, short or sees other keys, lengths
+    one off a tile's or a pair's edge, contexts that put the window's first tile anywhere."""
+    from vllm_kunlun_b200.ops.attention_cuda import paged_attention_cuda
+    from vllm_kunlun_b200.ops.gemm_cuda import check_status
+    spec = [(255, 255), (256, 256), (257, 257), (17, 1000), (129, 385), (384, 640), (640, 641), (100, 2149), (1100, 1100)]
+    seq_lens = [s for _, s in spec]
+    cache, bt = _make_paged(len(spec), seq_lens, Hkv, 128, 64, dtype=torch.bfloat16, seed=5)
+    qsl = torch.tensor([0] + list(torch.tensor([q for q, _ in spec]).cumsum(0)), dtype=torch.int32)
+    q = torch.randn(int(qsl[-1]), Hq, 128, generator=torch.Generator().manual_seed(9)).bfloat16()
+    q[::7] *= 6        # rows whose running maximum moves from tile to tile
+    sl = torch.tensor(seq_lens, dtype=torch.int32)
+    ref = ra.paged_attention(q, cache, bt, sl, qsl, 128 ** -0.5, window or None)
+    out = torch.full(q.shape, float("nan"), device=DEV, dtype=torch.bfloat16)
+    paged_attention_cuda(out, q.to(DEV), cache.to(DEV), bt.to(DEV), sl.to(DEV), qsl.to(DEV), 128 ** -0.5, 1100, 2149,
+                         window or None)
+    torch.cuda.synchronize()
+    check_status()
+    # weights and outputs in 16 bits: 2^-8 of values up to 4 standard deviations
+    _close(out, ref, 2e-2, 2e-2, f"prefill pairs window={window}")
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("T,N,K,group,splits", [(1, 256, 512, 128, 0), (16, 300, 1024, 64, 0), (16, 4096, 4096, 128, 0),
                                                 (32, 1024, 2048, 128, 0), (5, 384, 4096, 128, 4), (16, 128, 4096, 4096, 8),

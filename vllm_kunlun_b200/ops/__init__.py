@@ -492,7 +492,7 @@ def mla_prefill_attention(q, kv, k_pe, kv_starts, kv_lens, query_start_loc, caus
     gathered and up-projected chunk of cached context, not causal): ``q [T, N, 192]``, ``kv [rows, N * 256]``,
     ``k_pe [rows, 64]`` -> ``out [T, N, 128]``, natural-log ``lse [T, N]``.  Rows of requests without keys give
     zeros and ``-inf``.  Causal calls may carry a sliding ``window`` and ``sinks [N]`` (fp32); ``gate [T, N]`` multiplies
-    every head's output by its sigmoid.  CUDA: the tcgen05 prefill kernel (``csrc/attention/prefill_umma.cu``, MLA
+    every head's output by its sigmoid.  CUDA: the tcgen05 prefill kernel (``csrc/attention/prefill_pair.cu``, MLA
     instantiation)."""
     if q.is_cuda:
         T, N, _ = q.shape
