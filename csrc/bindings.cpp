@@ -1399,10 +1399,20 @@ void gdn_recurrent(at::Tensor out, const at::Tensor& q, const at::Tensor& k, con
   TORCH_CHECK(q.dim() == 3 && q.stride(2) == 1 && q.stride(1) == q.size(2) && k.stride(0) == q.stride(0) &&
               k.stride(1) == k.size(2) && v.stride(2) == 1 && v.stride(1) == v.size(2) && out.stride(1) == out.size(2));
   TORCH_CHECK(states.scalar_type() == at::kFloat && states.is_contiguous() && g.is_contiguous() && beta.is_contiguous());
+  c10::cuda::CUDAGuard guard(q.device());
+  GemmState& gs = gemm_state();
+  std::lock_guard<std::mutex> lk(gs.mu);
+  if (gs.num_sms == 0) {
+    gs.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+    gs.ws = at::empty({16 << 20}, q.options().dtype(at::kFloat));
+    gs.counters = at::zeros({1 << 16}, q.options().dtype(at::kInt));
+    gs.status = at::zeros({1}, q.options().dtype(at::kInt));
+  }
   check(b200_gdn_recurrent(out.data_ptr(), out.stride(0), q.data_ptr(), k.data_ptr(), q.stride(0), v.data_ptr(), v.stride(0),
                            g.data_ptr<float>(), beta.data_ptr<float>(), states.data_ptr<float>(), cu.data_ptr<int>(),
                            slots.data_ptr<int>(), (const uint8_t*)has_init.data_ptr(), (int)slots.size(0), (int)q.size(1),
-                           (int)v.size(1), (int)q.size(2), (int)v.size(2), (float)scale, l2norm, dtype_code(q), stream()),
+                           (int)v.size(1), (int)q.size(2), (int)v.size(2), (float)scale, l2norm, dtype_code(q), q.size(0),
+                           gs.status.data_ptr<int>(), stream()),
         "gdn_recurrent");
 }
 

@@ -10,7 +10,14 @@
 #include "../common/launch.cuh"
 #include "../common/utils.cuh"
 
+#include <limits.h>
+
 namespace b200 {
+// gdn_chunk.cu
+int gdn_chunk(void* out, int64_t o_stride, const void* q, const void* k, int64_t qk_stride, const void* v, int64_t v_stride,
+              const float* g, const float* beta, float* states, const int* cu, const int* slots, const uint8_t* has_init,
+              int64_t T, int R, int Hk, int Hv, float scale, int min_len, int* status, cudaStream_t st);
+
 namespace {
 
 // fp32 tensors keep full fp32 accuracy (this file is compiled without fast-math); 16-bit outputs use the fast forms
@@ -193,13 +200,17 @@ __global__ void gdn_gating_kernel(float* __restrict__ g, float* __restrict__ bet
 // share of the next chunk's q / k / v / g / beta in registers, so global-memory latency never sits on the
 // recurrence and the block synchronises twice per chunk instead of once per token.
 constexpr int kGdnChunk = 16;
+// New tokens of a request from which gdn_chunk.cu takes it.  While every head has an SM of its own the scan costs 10 us + 0.5 us a
+// token and 64 tokens in chunk form 21 us (one request of 24 / 48 / 64 tokens, 32 heads: scan 18.0 / 27.5 / 35.7 us); with more
+// heads than SMs the scan's blocks share them (8 requests of 24 tokens: scan 62.6 us, chunk form 44).
+constexpr int kGdnChunkMin = 40, kGdnChunkMinMany = 16;
 
 template <typename T, int DK>
 __global__ void __launch_bounds__(128) gdn_recurrent_kernel(
     T* __restrict__ out, int64_t o_stride, const T* __restrict__ q, const T* __restrict__ k, int64_t qk_stride,
     const T* __restrict__ v, int64_t v_stride, const float* __restrict__ g, const float* __restrict__ beta,
     float* __restrict__ states /*[slots, Hv, Dv, DK]*/, const int* __restrict__ cu, const int* __restrict__ slots,
-    const uint8_t* __restrict__ has_init, int Hk, int Hv, int Dv, float scale, int l2norm) {
+    const uint8_t* __restrict__ has_init, int Hk, int Hv, int Dv, float scale, int l2norm, int chunk_min) {
   static_assert(DK % 16 == 0 && DK <= 128, "DK");
   constexpr int QW = DK / 4;                      // state columns per thread
   constexpr int CH = kGdnChunk;
@@ -213,7 +224,7 @@ __global__ void __launch_bounds__(128) gdn_recurrent_kernel(
   const int hv = blockIdx.y, r = blockIdx.z, hk = hv / (Hv / Hk);
   const int row0 = blockIdx.x * 32, row = row0 + rl;
   const int s = cu[r], L = cu[r + 1] - s, slot = slots[r];
-  if (L == 0 || slot < 0) return;
+  if (L == 0 || L >= chunk_min || slot < 0) return;
   // Column ownership is interleaved in 16-byte pieces: registers S[4i .. 4i+3] of quarter qd hold columns
   // 16 i + 4 qd .. + 3, so that the four quarter-lanes of a row read four consecutive float4 of the shared k / q row
   // (distinct banks) instead of four addresses 128 bytes apart (one bank, a 4-way conflict on every load).
@@ -420,14 +431,27 @@ extern "C" int b200_gdn_gating(float* g, float* beta, const void* a, int64_t a_s
 extern "C" int b200_gdn_recurrent(void* out, int64_t o_stride, const void* q, const void* k, int64_t qk_stride, const void* v,
                                   int64_t v_stride, const float* g, const float* beta, float* states, const int* cu,
                                   const int* slots, const uint8_t* has_init, int R, int Hk, int Hv, int Dk, int Dv, float scale,
-                                  int l2norm, int dtype, cudaStream_t st) {
+                                  int l2norm, int dtype, int64_t T_, int* status, cudaStream_t st) {
   if (R == 0) return 0;
   if (Dv % 32 != 0 || Hv % Hk != 0) return 3;
+  // Prompts go through the chunked form (4 x 2048 tokens, 32 heads: 3308 us as a scan, 221 us).  Normalised q and k only: the
+  // inverse that it needs is of a matrix whose entries the norms bound.  T_ - (R - 1) rows are the most that one request can have
+  // when each of the others has a row: decode steps go straight to the scan.
+  const int min_len = (int64_t)R * Hv > 148 ? b200::kGdnChunkMinMany : b200::kGdnChunkMin;
+  int chunk_min = INT_MAX;
+  if (dtype == b200::kBF16 && l2norm && Dk == 128 && Dv == 128 && T_ - (R - 1) >= min_len) {
+    chunk_min = R == 1 ? 1 : min_len;   // a lone request needs no second launch
+    const int rc = b200::gdn_chunk(out, o_stride, q, k, qk_stride, v, v_stride, g, beta, states, cu, slots, has_init, T_, R, Hk,
+                                   Hv, scale, chunk_min, status, st);
+    if (rc > 0) return rc;
+    if (rc == 0 && R == 1) return 0;
+    if (rc < 0) chunk_min = INT_MAX;
+  }
   dim3 grid(Dv / 32, Hv, R);
 #define B200_GDN_LAUNCH(DK)                                                                                          \
   B200_DISPATCH_DTYPE(dtype, (b200::gdn_recurrent_kernel<T, DK><<<grid, 128, 0, st>>>(                                  \
                                  (T*)out, o_stride, (const T*)q, (const T*)k, qk_stride, (const T*)v, v_stride, g, beta, \
-                                 states, cu, slots, has_init, Hk, Hv, Dv, scale, l2norm)))
+                                 states, cu, slots, has_init, Hk, Hv, Dv, scale, l2norm, chunk_min)))
   if (Dk == 128) { B200_GDN_LAUNCH(128); }
   else if (Dk == 64) { B200_GDN_LAUNCH(64); }
   else if (Dk == 32) { B200_GDN_LAUNCH(32); }

@@ -150,6 +150,35 @@ def test_gated_delta_rule_varlen(Dk, Dv, Hk, Hv):
     torch.testing.assert_close(s_dev.cpu(), s_ref, atol=2e-3, rtol=2e-3)
 
 
+@pytest.mark.parametrize("lens,Hk,Hv,offset", [([1], 1, 1, 0), ([40], 1, 2, 0), ([64], 2, 2, 0), ([65, 0, 1, 63], 1, 2, 0),
+                                               ([39, 128, 191, 7], 2, 4, 0), ([193, 16, 15, 40, 1], 16, 32, 0), ([130], 1, 2, 4)])
+def test_gated_delta_rule_chunk_edges(lens, Hk, Hv, offset):
+    """Requests around the lengths at which the chunk kernel takes over from the scan and around its chunks of 64 tokens, without
+    rows, without a state slot, with and without a carried state; ``offset``: rows that no tensor map can read.  Both routes keep
+    fp32 throughout: states agree to 2^-24 times the square root of the steps, with a factor of 30 for the sums of 128 terms and
+    the state's cancellations (1e-4); outputs to the rounding of bf16 (2^-8 of the value) beside that."""
+    torch.manual_seed(11)
+    T, R, C = sum(lens), len(lens), (2 * Hk + Hv) * 128
+    wide = torch.randn(T, C + 8).to(torch.bfloat16)
+    g, beta = -torch.rand(T, Hv) * torch.tensor([0.02, 1.0])[torch.arange(Hv) % 2], torch.rand(T, Hv)
+    states = torch.randn(R + 2, Hv, 128, 128) * 0.1
+    slots = torch.randperm(R + 2)[:R].to(torch.int32)
+    if R > 3:
+        slots[-1] = -1
+    init = (torch.arange(R) % 2).to(torch.int32)
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32)
+
+    def run(dev):
+        m, st = wide.to(dev)[:, offset:offset + C], states.to(dev)
+        q, k, v = (m[:, a * 128:b * 128].view(T, b - a, 128) for a, b in ((0, Hk), (Hk, 2 * Hk), (2 * Hk, 2 * Hk + Hv)))
+        return ops.gated_delta_rule(q, k, v, g.to(dev), beta.to(dev), st, cu.to(dev), slots.to(dev), init.to(dev)).cpu(), st.cpu()
+
+    (got, got_st), (want, want_st) = run(DEV), run("cpu")
+    torch.testing.assert_close(got_st, want_st, atol=1e-4, rtol=1e-4)
+    n = T - (lens[-1] if R > 3 else 0)
+    torch.testing.assert_close(got[:n].float(), want[:n].float(), atol=1e-3, rtol=2 ** -7)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("pattern", ["random", "segments"])
 @pytest.mark.parametrize("N,offset,r", [(640, 128, 16), (333, 5, 8), (1030, 0, 12)])
