@@ -104,6 +104,11 @@ typedef struct GroupedGemmArgs {
   int bn;                // token tile 16 / 32 / 64 / 128
   int grid;
   int act;               // 0, or 4 = square of relu (16-bit inputs)
+  // fp8 with bn = 128, or null: out is e4m3(act(gate) * up) [M, N / 2] with these scales [N / 256, out_stride], gate and up
+  // being the two halves of the weight rows; out_fmt: the type that gate, up and the product are rounded to
+  float* out_scale;
+  int out_stride;
+  int fused_act;         // 0 silu, 1 gelu (tanh form)
 } GroupedGemmArgs;
 int b200_grouped_gemm_launch(const GroupedGemmArgs* a, const void* tmapW, const void* tmapX, cudaStream_t st);
 
@@ -228,6 +233,9 @@ int b200_topk_rows(int* out, const float* logits, const int* row_len, int64_t ro
 int b200_moe_route(float* out_w, int* out_ids, const void* logits, const float* bias, int64_t T, int E, int k, int mode,
                    int renorm, int n_group, int topk_group, int group_top, float scale, int64_t stride, int dtype,
                    cudaStream_t st);
+int b200_moe_permute_quant(void* q_sorted, float* scale_t, int64_t s_stride, int* pos_of_pair, int* lod, int* counts, int* cursor,
+                           const void* x, const int* ids, const int* emap, int64_t T_, int k, int H, int E_local, int E_global,
+                           int64_t x_stride, int dtype, cudaStream_t st);
 int b200_moe_permute(void* x_sorted, int* pos_of_pair, int* lod, int* counts, int* cursor, const void* x, const int* ids,
                      const int* emap, const float* factors, int64_t T, int k, int H, int E_local, int E_global,
                      int64_t x_stride, int64_t max_rows, int dtype, cudaStream_t st);  // factors [T][k] (or null): times the rows

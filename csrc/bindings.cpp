@@ -579,18 +579,26 @@ c10::optional<at::Tensor> gemm_status_tensor() {
 }
 void gemm_clear_tmap_cache() { gemm_state().cache.clear(); }
 
+// Token tile of a grouped GEMM: rows per group decide, decode batches spread thin over many experts.
+int grouped_bn(bool grouped, int M, int E) {
+  const int per_group = grouped ? std::max(1, M / std::max(1, E / 4)) : M;
+  return per_group <= 16 ? 16 : per_group <= 32 ? 32 : per_group <= 64 ? 64 : 128;
+}
+
 // out[M, N] = x[M, K] @ w[e(row)]^T for rows sorted by expert (lod), or one group when lod is absent.
 // fp8: x / w are uint8 views of e4m3 data, a_scale_t [K/128, stride], w_scale [E, N/128, K/128].
-void grouped_gemm(at::Tensor out, const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& lod,
-                  const c10::optional<at::Tensor>& bias, const c10::optional<at::Tensor>& a_scale_t,
-                  const c10::optional<at::Tensor>& w_scale, int64_t bn, int64_t act) {
+// `out_scale` (fp8, bn = 128): out [M, N / 2] = e4m3 of act(gate) * up, see GroupedGemmArgs.
+void grouped_gemm_impl(at::Tensor out, const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& lod,
+                       const c10::optional<at::Tensor>& bias, const c10::optional<at::Tensor>& a_scale_t,
+                       const c10::optional<at::Tensor>& w_scale, int64_t bn, int64_t act, const at::Tensor* out_scale,
+                       at::ScalarType round_type) {
   TORCH_CHECK(x.is_cuda() && w.is_cuda() && x.dim() == 2 && (w.dim() == 3 || w.dim() == 2));
   TORCH_CHECK(x.stride(1) == 1 && w.is_contiguous() && out.stride(1) == 1);
   const bool fp8 = x.element_size() == 1;
   TORCH_CHECK(w.element_size() == x.element_size());
   const int E = w.dim() == 3 ? w.size(0) : 1;
   const int N = w.size(-2), K = w.size(-1), M = x.size(0);
-  TORCH_CHECK(x.size(1) == K && out.size(0) == M && out.size(1) == N);
+  TORCH_CHECK(x.size(1) == K && out.size(0) == M && out.size(1) == (out_scale ? N / 2 : N));
   TORCH_CHECK((K * x.element_size()) % 16 == 0 && (x.stride(0) * x.element_size()) % 16 == 0);
   if (M == 0) return;
   if (fp8) TORCH_CHECK(a_scale_t.has_value() && w_scale.has_value() && a_scale_t->stride(1) == 1 && w_scale->is_contiguous());
@@ -604,6 +612,7 @@ void grouped_gemm(at::Tensor out, const at::Tensor& x, const at::Tensor& w, cons
     gs.status = at::zeros({1}, x.options().dtype(at::kInt));
   }
   GroupedGemmArgs a;
+  memset(&a, 0, sizeof(a));
   a.out = out.data_ptr(); a.bias = opt_ptr(bias);
   a.lod = lod.has_value() ? lod->data_ptr<int>() : nullptr;
   a.a_scale = fp8 ? a_scale_t->data_ptr<float>() : nullptr;
@@ -611,24 +620,50 @@ void grouped_gemm(at::Tensor out, const at::Tensor& x, const at::Tensor& w, cons
   a.status = gs.status.data_ptr<int>();
   a.M = M; a.N = N; a.K = K; a.E = E; a.ldo = out.stride(0);
   a.a_stride = fp8 ? a_scale_t->stride(0) : 0;
-  a.fp8 = fp8; a.fmt = x.scalar_type() == at::kBFloat16 ? 1 : 0; a.out_fmt = out.scalar_type() == at::kBFloat16 ? 1 : out.scalar_type() == at::kFloat ? 2 : 0;
+  a.fp8 = fp8; a.fmt = x.scalar_type() == at::kBFloat16 ? 1 : 0; a.out_fmt = round_type == at::kBFloat16 ? 1 : round_type == at::kFloat ? 2 : 0;
   if (a.out_fmt == 2) TORCH_CHECK(!fp8 && !bias.has_value(), "fp32 output: 16-bit inputs, no bias");
-  int b = (int)bn;
-  if (b <= 0) {
-    // rows per group decide the token tile: decode batches spread thin over many experts
-    int per_group = lod.has_value() ? std::max(1, M / std::max(1, E / 4)) : M;
-    b = per_group <= 16 ? 16 : per_group <= 32 ? 32 : per_group <= 64 ? 64 : 128;
+  if (out_scale != nullptr) {
+    a.out_scale = out_scale->data_ptr<float>();
+    a.out_stride = out_scale->stride(0);
+    a.fused_act = (int)act;
+    act = 0;
   }
+  const int b = bn > 0 ? (int)bn : grouped_bn(lod.has_value(), M, E);
   a.bn = b;
   a.act = (int)act;
-  int64_t n_tiles = (N + 127) / 128;
+  const bool wide = fp8 && b == 128;   // tiles of 128 rows x 256 weight rows
+  const int64_t n_tiles = wide ? (N + 255) / 256 : (N + 127) / 128;
   int64_t max_tiles = n_tiles * ((M + b - 1) / b + (lod.has_value() ? E : 0));
   a.grid = (int)std::min<int64_t>(max_tiles, (int64_t)gs.num_sms * (b <= 64 ? 2 : 1));
   at::Tensor w2 = w.dim() == 3 ? w.view({(int64_t)E * N, K}) : w;
   const int eb = x.element_size();
   const Tmap& tw = get_tmap(gs, w2, 128, eb);
-  const Tmap& tx = get_tmap(gs, x, b, eb);
+  const Tmap& tx = get_tmap(gs, x, wide ? 64 : b, eb);
   check(b200_grouped_gemm_launch(&a, tw.b, tx.b, stream()), "grouped gemm launch");
+}
+
+void grouped_gemm(at::Tensor out, const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& lod,
+                  const c10::optional<at::Tensor>& bias, const c10::optional<at::Tensor>& a_scale_t,
+                  const c10::optional<at::Tensor>& w_scale, int64_t bn, int64_t act) {
+  grouped_gemm_impl(out, x, w, lod, bias, a_scale_t, w_scale, bn, act, nullptr, out.scalar_type());
+}
+
+// (q uint8 [M, I], scale_t [I/128, stride]) = fp8(act(x Wg^T) * (x Wu^T)) of fp8 rows sorted by expert, `w` [E, 2 I, K] = gate
+// rows, then up rows; an empty list where the two-kernel path is to be taken: narrow tiles, I no multiple of 128.
+std::vector<at::Tensor> grouped_gemm_act_fp8(const at::Tensor& x, const at::Tensor& w, const at::Tensor& lod,
+                                             const c10::optional<at::Tensor>& bias, const at::Tensor& a_scale_t,
+                                             const at::Tensor& w_scale, int64_t act, const at::Tensor& like) {
+  const int64_t M = x.size(0), I = w.size(1) / 2;
+  const at::ScalarType model_type = like.scalar_type();
+  if (w.size(1) % 256 != 0 || M == 0 || grouped_bn(true, (int)M, (int)w.size(0)) != 128 ||
+      (model_type != at::kBFloat16 && model_type != at::kHalf))
+    return {};
+  TORCH_CHECK(x.element_size() == 1 && w.dim() == 3 && (act == 0 || act == 1));
+  const int64_t stride = std::max<int64_t>(4, (M + 3) / 4 * 4);
+  auto q = at::empty({M, I}, x.options().dtype(at::kByte));
+  auto s = at::empty({I / 128, stride}, x.options().dtype(at::kFloat));
+  grouped_gemm_impl(q, x, w, lod, bias, a_scale_t, w_scale, 128, act, &s, model_type);
+  return {q, s};
 }
 
 std::vector<at::Tensor> moe_route(const at::Tensor& logits, const c10::optional<at::Tensor>& bias, int64_t k,
@@ -669,6 +704,28 @@ std::vector<at::Tensor> moe_permute(const at::Tensor& x, const at::Tensor& ids, 
                          x.stride(0), max_rows, dtype_code(x), stream()),
         "moe_permute", 3);
   return {xs, pos, lod};
+}
+
+// The same with the rows as e4m3: returns q_sorted [T*k, H] uint8, scale_t [H/128, stride], pos_of_pair, lod; an empty list for
+// rows that it does not serve (fp32, unaligned, H no multiple of 128, more than 16 experts a token).
+std::vector<at::Tensor> moe_permute_quant(const at::Tensor& x, const at::Tensor& ids, const c10::optional<at::Tensor>& emap,
+                                          int64_t E_local, int64_t E_global, at::Tensor state) {
+  TORCH_CHECK(x.dim() == 2 && x.stride(1) == 1 && ids.is_contiguous() && ids.scalar_type() == at::kInt);
+  TORCH_CHECK(state.scalar_type() == at::kInt && state.numel() >= 2 * E_local);
+  const int64_t T = x.size(0), k = ids.size(1), H = x.size(1), M = T * k;
+  if (x.element_size() != 2 || H % 128 != 0 || k > 16 || M == 0 || x.stride(0) % 8 != 0 || ((uintptr_t)x.data_ptr() & 15) != 0)
+    return {};
+  const int64_t stride = std::max<int64_t>(4, (M + 3) / 4 * 4);
+  auto q = at::empty({M, H}, x.options().dtype(at::kByte));
+  auto st = at::empty({H / 128, stride}, x.options().dtype(at::kFloat));
+  auto pos = at::empty({M}, ids.options());
+  auto lod = at::empty({E_local + 1}, ids.options());
+  check(b200_moe_permute_quant(q.data_ptr(), st.data_ptr<float>(), stride, pos.data_ptr<int>(), lod.data_ptr<int>(),
+                               state.data_ptr<int>(), state.data_ptr<int>() + E_local, x.data_ptr(), ids.data_ptr<int>(),
+                               emap.has_value() ? emap->data_ptr<int>() : nullptr, T, (int)k, (int)H, (int)E_local, (int)E_global,
+                               x.stride(0), dtype_code(x), stream()),
+        "moe_permute_quant", 3);
+  return {q, st, pos, lod};
 }
 
 // (weights [T, k] fp32, ids [T, k] int32) straight from the hidden states: router GEMM + routing in one launch
@@ -1996,10 +2053,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_int8", &gemm_int8);
   m.def("quant_int8_token", &quant_int8_token);
   m.def("set_gemm_decode_comm", &set_gemm_decode_comm);
+  m.def("grouped_gemm_act_fp8", &grouped_gemm_act_fp8);
   m.def("grouped_gemm", &grouped_gemm, py::arg("out"), py::arg("x"), py::arg("w"), py::arg("lod"), py::arg("bias"),
         py::arg("a_scale_t"), py::arg("w_scale"), py::arg("bn"), py::arg("act") = 0);
   m.def("moe_route", &moe_route, py::arg("logits"), py::arg("bias"), py::arg("k"), py::arg("mode"), py::arg("renorm"),
         py::arg("n_group"), py::arg("topk_group"), py::arg("scale"), py::arg("group_top") = 2);
+  m.def("moe_permute_quant", &moe_permute_quant);
   m.def("moe_permute", &moe_permute, py::arg("x"), py::arg("ids"), py::arg("emap"), py::arg("E_local"),
         py::arg("E_global"), py::arg("state"), py::arg("max_rows") = 0, py::arg("factors") = py::none());
   m.def("moe_unpermute", &moe_unpermute);

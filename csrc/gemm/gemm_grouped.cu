@@ -342,11 +342,17 @@ static cudaError_t launch_grouped(const GroupedGemmArgs& a, const CUtensorMap& t
 
 }  // namespace b200
 
+namespace b200 {
+// gemm_grouped_fp8.cu: fp8 inputs with more than a few rows a group
+int grouped_fp8_launch(const GroupedGemmArgs& a, const CUtensorMap& tmW, const CUtensorMap& tmX, cudaStream_t st);
+}  // namespace b200
+
 extern "C" int b200_grouped_gemm_launch(const GroupedGemmArgs* a, const void* tmW, const void* tmX, cudaStream_t st) {
   using namespace b200;
   if (a->E > kGMaxExperts || (a->act != 0 && (a->act != kRelu2 || a->fp8))) return 2;
   const CUtensorMap& w = *reinterpret_cast<const CUtensorMap*>(tmW);
   const CUtensorMap& x = *reinterpret_cast<const CUtensorMap*>(tmX);
+  if (a->fp8 && a->bn == 128) return grouped_fp8_launch(*a, w, x, st);
   cudaError_t e = cudaErrorInvalidValue;
 #define B200_G_CASE(BN_)                                                                                     \
   case BN_:                                                                                                  \
@@ -360,7 +366,11 @@ extern "C" int b200_grouped_gemm_launch(const GroupedGemmArgs* a, const void* tm
     B200_G_CASE(16)
     B200_G_CASE(32)
     B200_G_CASE(64)
-    B200_G_CASE(128)
+    case 128:
+      if (a->out_fmt == 2) e = launch_grouped<128, false, float>(*a, w, x, st);
+      else e = (a->fmt == 1) ? launch_grouped<128, false, __nv_bfloat16>(*a, w, x, st)
+                             : launch_grouped<128, false, __half>(*a, w, x, st);
+      break;
     default: break;
   }
 #undef B200_G_CASE

@@ -179,6 +179,77 @@ def test_gated_delta_rule_chunk_edges(lens, Hk, Hv, offset):
     torch.testing.assert_close(got[:n].float(), want[:n].float(), atol=1e-3, rtol=2 ** -7)
 
 
+@pytest.mark.parametrize("rows", [[300, 0, 1, 63, 64, 65], [127, 128, 129, 257]])
+@pytest.mark.parametrize("N,K,bias", [(512, 256, False), (384, 128, True), (200, 384, False)])
+def test_grouped_fp8_wide_tiles(rows, N, K, bias):
+    """128-row tiles of the fp8 grouped GEMM: empty, short and ragged groups, an odd number of weight blocks, columns off the 16-byte
+    stores.  The products of a k-block are exact in 64 bits and summed in fp32 on the GPU: K / 128 + 128 roundings of 2^-24, far
+    below the output's 2^-9, so the tolerance is that of bf16; groups without rows write nothing."""
+    from vllm_kunlun_b200.ops import _ext
+    torch.manual_seed(13)
+    C, E, M = _ext.C(), len(rows), sum(rows)
+    x = torch.randn(M, K, device=DEV).to(torch.float8_e4m3fn)
+    w = torch.randn(E, N, K, device=DEV).to(torch.float8_e4m3fn)
+    nb, kb = -(-N // 128), K // 128
+    a_s, w_s = torch.rand(kb, (M + 3) // 4 * 4, device=DEV) + 0.1, torch.rand(E, nb, kb, device=DEV) + 0.1
+    b = torch.randn(E, N, device=DEV).bfloat16() if bias else None
+    lod = torch.tensor([0] + rows, device=DEV).cumsum(0).int()
+    out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    C.grouped_gemm(out, x.view(torch.uint8), w.view(torch.uint8), lod, b, a_s, w_s, 128)
+    want = torch.zeros(M, N, dtype=torch.float64, device=DEV)
+    for e in range(E):
+        r = slice(int(lod[e]), int(lod[e + 1]))
+        for i in range(kb):
+            c = slice(128 * i, 128 * i + 128)
+            want[r] += (x[r, c].double() @ w[e, :, c].double().T) * a_s[i, r, None].double() * w_s[e, :, i].double().repeat_interleave(128)[:N]
+        if bias:
+            want[r] += b[e].double()
+    torch.testing.assert_close(out.double(), want, atol=1e-2, rtol=2 ** -8)
+
+
+@pytest.mark.parametrize("act", [0, 1])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_grouped_fp8_with_activation(act, dtype):
+    """Activation and quantiser in the epilogue of the first expert GEMM: the bytes and scales of the kernels that it replaces."""
+    from vllm_kunlun_b200.ops import _ext
+    torch.manual_seed(14)
+    C, rows, inter, K = _ext.C(), [130, 1, 0, 64, 200], 256, 384
+    E, M = len(rows), sum(rows)
+    x = torch.randn(M, K, device=DEV).to(torch.float8_e4m3fn).view(torch.uint8)
+    w = torch.randn(E, 2 * inter, K, device=DEV).to(torch.float8_e4m3fn).view(torch.uint8)
+    a_s, w_s = torch.rand(K // 128, (M + 3) // 4 * 4, device=DEV) * 0.02, torch.rand(E, 2 * inter // 128, K // 128, device=DEV)
+    b = torch.randn(E, 2 * inter, device=DEV).to(dtype)
+    lod = torch.tensor([0] + rows, device=DEV).cumsum(0).int()
+    h = torch.empty(M, 2 * inter, dtype=dtype, device=DEV)
+    C.grouped_gemm(h, x, w, lod, b, a_s, w_s, 128)
+    want_q, want_s = C.act_mul_quant_fp8(h, act, lod[E:])
+    q, s = C.grouped_gemm_act_fp8(x, w, lod, b, a_s, w_s, act, h)
+    assert torch.equal(q, want_q) and torch.equal(s[:, :M], want_s[:, :M])
+
+
+@pytest.mark.parametrize("T,k,H,mapped", [(129, 8, 256, False), (300, 4, 2048 + 128, True)])
+def test_moe_permute_quant(T, k, H, mapped):
+    """Rows quantised on their way to their experts: every pair's row is the quantised row of its token, pairs of other ranks' experts
+    have no place, and the places are those of the segments."""
+    from vllm_kunlun_b200.ops import _ext
+    torch.manual_seed(15)
+    C, E = _ext.C(), 16
+    x = torch.randn(T, H, device=DEV).bfloat16()
+    ids = torch.rand(T, E, device=DEV).topk(k, -1).indices.int()
+    emap = torch.where(torch.arange(E, device=DEV) % 2 == 0, torch.arange(E, device=DEV) // 2, -1).int() if mapped else None
+    local = E // 2 if mapped else E
+    q, st, pos, lod = C.moe_permute_quant(x, ids, emap, local, E, torch.zeros(2 * local, dtype=torch.int32, device=DEV))
+    want_q, want_s = C.quant_fp8_group(x, False, None, 4)
+    where = emap[ids.long()].flatten() if mapped else ids.flatten()
+    assert torch.equal(pos < 0, where < 0)
+    pair = (where >= 0).nonzero()[:, 0]
+    p, token = pos[pair].long(), pair // k
+    assert torch.equal(q[p], want_q[token]) and torch.equal(st[:, p], want_s[:, token])
+    assert p.unique().numel() == pair.numel() == int(lod[-1])
+    e = where[pair].long()
+    assert bool(((p >= lod[e]) & (p < lod[e + 1])).all())
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("pattern", ["random", "segments"])
 @pytest.mark.parametrize("N,offset,r", [(640, 128, 16), (333, 5, 8), (1030, 0, 12)])

@@ -1,7 +1,7 @@
 """CUDA MoE path: routing -> permute -> grouped GEMM -> act -> grouped GEMM -> weighted un-permute.
 
 Kernels: ``csrc/moe/moe.cu`` (route / count / scan / scatter / un-permute / fp8 quant) and
-``csrc/gemm/gemm_grouped.cu`` (tcgen05 grouped GEMM, bf16 or fp8 block-scaled).  All shapes are
+``csrc/gemm/gemm_grouped{,_fp8}.cu`` (tcgen05 grouped GEMM, bf16 or fp8 block-scaled).  All shapes are
 static in the token count (``T * k`` permuted rows, invalid rows masked by ``lod``), so the whole
 block can sit inside a captured CUDA graph."""
 from __future__ import annotations
@@ -51,23 +51,34 @@ def fused_moe_cuda(x, w13, w2, topk_weights, topk_ids, act="silu", b13=None, b2=
         xs, pos, lod, st = C.moe_prepare_small(x, topk_ids.contiguous(), expert_map, E_local, E_global, fp8)
         q = xs
     else:
-        xs, pos, lod = C.moe_permute(x, topk_ids.contiguous(), expert_map, E_local, E_global, _state(x.device, E_local))
-        if fp8:
-            q, st = C.quant_fp8_group(xs, False, lod[E_local:], 4)
+        ids, state = topk_ids.contiguous(), _state(x.device, E_local)
+        done = C.moe_permute_quant(x, ids, expert_map, E_local, E_global, state) if fp8 else None
+        if done:
+            q, st, pos, lod = done
+            xs = q
+        else:
+            xs, pos, lod = C.moe_permute(x, ids, expert_map, E_local, E_global, state)
+            if fp8:
+                q, st = C.quant_fp8_group(xs, False, lod[E_local:], 4)
     M = xs.shape[0]
-    h = torch.empty(M, w13.shape[1], dtype=x.dtype, device=x.device)
-    if fp8:
-        C.grouped_gemm(h, q, w13.view(torch.uint8), lod, b13, st, w13_scale, 0)
-    else:
-        C.grouped_gemm(h, xs, w13, lod, b13, None, None, 0)
     y = torch.empty(M, H, dtype=x.dtype, device=x.device)
     if fp8:
-        if act in ("silu", "gelu_tanh") and SMALL_BATCH_FUSION[0]:
-            q2, st2 = C.act_mul_quant_fp8(h, 0 if act == "silu" else 1, lod[E_local:])  # activation + quantiser fused
+        fuse, code = act in ("silu", "gelu_tanh") and SMALL_BATCH_FUSION[0], 0 if act == "silu" else 1
+        # many rows an expert: activation and quantiser in the first GEMM's epilogue
+        done = C.grouped_gemm_act_fp8(q, w13.view(torch.uint8), lod, b13, st, w13_scale, code, x) if fuse else None
+        if done:
+            q2, st2 = done
         else:
-            q2, st2 = C.quant_fp8_group(act_and_mul(h, act), False, lod[E_local:], 4)
+            h = torch.empty(M, w13.shape[1], dtype=x.dtype, device=x.device)
+            C.grouped_gemm(h, q, w13.view(torch.uint8), lod, b13, st, w13_scale, 0)
+            if fuse:
+                q2, st2 = C.act_mul_quant_fp8(h, code, lod[E_local:])  # activation + quantiser fused
+            else:
+                q2, st2 = C.quant_fp8_group(act_and_mul(h, act), False, lod[E_local:], 4)
         C.grouped_gemm(y, q2, w2.view(torch.uint8), lod, b2, st2, w2_scale, 0)
     else:
+        h = torch.empty(M, w13.shape[1], dtype=x.dtype, device=x.device)
+        C.grouped_gemm(h, xs, w13, lod, b13, None, None, 0)
         C.grouped_gemm(y, act_and_mul(h, act), w2, lod, b2, None, None, 0)
     out = torch.empty(T, H, dtype=x.dtype, device=x.device)
     C.moe_unpermute(out, y, pos, topk_weights.contiguous())
