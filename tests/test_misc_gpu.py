@@ -179,6 +179,29 @@ def test_gated_delta_rule_chunk_edges(lens, Hk, Hv, offset):
     torch.testing.assert_close(got[:n].float(), want[:n].float(), atol=1e-3, rtol=2 ** -7)
 
 
+@pytest.mark.parametrize("lens,Hk,Hv,Dv,dtype", [([1] * 5, 2, 4, 128, torch.bfloat16), ([2, 0, 1, 3], 1, 2, 64, torch.float16),
+                                                 ([1, 1, 2], 2, 2, 32, torch.float32)])
+@pytest.mark.parametrize("l2norm", [True, False])
+def test_gated_delta_rule_steps(lens, Hk, Hv, Dv, dtype, l2norm):
+    """A row or two a request (also none, and three): the decode kernel against the oracle.  Both in fp32 on the same inputs: states
+    to 2^-24 times the 128 terms of a sum (1e-5), outputs to the rounding of their type beside that."""
+    torch.manual_seed(12)
+    T, R = sum(lens), len(lens)
+    q, k, v = (torch.randn(T, h, d).mul(0.2).to(dtype) for h, d in ((Hk, 128), (Hk, 128), (Hv, Dv)))
+    g, beta, states = -torch.rand(T, Hv), torch.rand(T, Hv), torch.randn(R + 1, Hv, Dv, 128) * 0.1
+    slots, init = torch.randperm(R + 1)[:R].to(torch.int32), (torch.arange(R) % 2).to(torch.int32)
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32)
+
+    def run(dev):
+        st = states.to(dev)
+        o = ops.gated_delta_rule(*(t.to(dev) for t in (q, k, v, g, beta)), st, cu.to(dev), slots.to(dev), init.to(dev), None, l2norm)
+        return o.cpu().float(), st.cpu()
+
+    (got, got_st), (want, want_st) = run(DEV), run("cpu")
+    torch.testing.assert_close(got_st, want_st, atol=1e-5, rtol=1e-5)
+    torch.testing.assert_close(got, want, atol=1e-5, rtol={torch.float32: 1e-4, torch.float16: 2 ** -9, torch.bfloat16: 2 ** -7}[dtype])
+
+
 @pytest.mark.parametrize("rows", [[300, 0, 1, 63, 64, 65], [127, 128, 129, 257]])
 @pytest.mark.parametrize("N,K,bias", [(512, 256, False), (384, 128, True), (200, 384, False)])
 def test_grouped_fp8_wide_tiles(rows, N, K, bias):
