@@ -35,9 +35,11 @@ __device__ __forceinline__ int find_seq(const int* __restrict__ cu, int R, int t
 
 // y[t, c] = act(bias[c] + sum_j w[c, j] * in[t - (W-1) + j, c]); positions before the sequence start read
 // the cached state (rows W-1+p.. of the previous inputs) or zero.
-// One thread = one 16-byte channel vector x kConvTok consecutive tokens, with a sliding window of the last W-1
-// input rows in registers, so every input row is loaded once per thread.
-constexpr int kConvTok = 8;
+// One thread = one 16-byte channel vector x kConvTok consecutive tokens, with a sliding window of the last W-1 input rows in
+// registers, so every input row is loaded once per thread; the loads of kConvBatch rows are in flight together.  Bound by
+// memory: 8192 tokens x 8192 channels are 268 MB (41 us); 89 us, and 140 with eight tokens
+// a thread, taps read one by one and one row in flight.
+constexpr int kConvTok = 16, kConvBatch = 8;
 
 template <typename T, int W>
 __global__ void __launch_bounds__(128) conv1d_fwd_kernel(T* __restrict__ out, int64_t out_stride, const T* __restrict__ x,
@@ -50,12 +52,20 @@ __global__ void __launch_bounds__(128) conv1d_fwd_kernel(T* __restrict__ out, in
   const int64_t t0 = (int64_t)blockIdx.y * kConvTok;
   if (c0 >= C || t0 >= Ttot) return;
   float wv[W][V], bv[V];
+  const T* wc = w + (int64_t)c0 * W;              // the V channels' taps are V * W consecutive numbers
+  if ((reinterpret_cast<uintptr_t>(w) & 15) == 0) {
 #pragma unroll
-  for (int e = 0; e < V; ++e) {
-    bv[e] = bias ? to_f(bias[c0 + e]) : 0.f;
+    for (int i = 0; i < W; ++i) {
+      const Vec16<T> a = ld_vec(wc + i * V);
 #pragma unroll
-    for (int j = 0; j < W; ++j) wv[j][e] = to_f(w[(int64_t)(c0 + e) * W + j]);
+      for (int e = 0; e < V; ++e) wv[(i * V + e) % W][(i * V + e) / W] = to_f(a.v[e]);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < W * V; ++i) wv[i % W][i / W] = to_f(wc[i]);
   }
+#pragma unroll
+  for (int e = 0; e < V; ++e) bv[e] = bias ? to_f(bias[c0 + e]) : 0.f;
   float win[W][V];  // win[j] = input row at (current token) - (W-1) + j
   int r = find_seq(cu, R, (int)t0);
   int seq_start = cu[r], seq_end = cu[r + 1];
@@ -81,28 +91,35 @@ __global__ void __launch_bounds__(128) conv1d_fwd_kernel(T* __restrict__ out, in
     }
   };
   load_hist(t0);
-  for (int i = 0; i < kConvTok; ++i) {
-    const int64_t t = t0 + i;
-    if (t >= Ttot) break;
-    if (t >= seq_end) {  // crossed into the next (non-empty) sequence: its history comes from its own state
-      while (t >= seq_end) { ++r; seq_start = cu[r]; seq_end = cu[r + 1]; }
-      load_hist(t);
-    }
-    Vec16<T> cur = ld_vec(x + t * x_stride + c0);
-    Vec16<T> o;
+#pragma unroll 1
+  for (int i0 = 0; i0 < kConvTok; i0 += kConvBatch) {
+    Vec16<T> rows[kConvBatch];
 #pragma unroll
-    for (int e = 0; e < V; ++e) {
-      win[W - 1][e] = to_f(cur.v[e]);
-      float acc = bv[e];
+    for (int i = 0; i < kConvBatch; ++i)
+      if (t0 + i0 + i < Ttot) rows[i] = ld_vec(x + (t0 + i0 + i) * x_stride + c0);
 #pragma unroll
-      for (int j = 0; j < W; ++j) acc += wv[j][e] * win[j][e];
-      o.v[e] = from_f<T>(act ? silu<T>(acc) : acc);
-    }
-    st_vec(out + t * out_stride + c0, o);
+    for (int i = 0; i < kConvBatch; ++i) {
+      const int64_t t = t0 + i0 + i;
+      if (t >= Ttot) return;
+      if (t >= seq_end) {  // crossed into the next (non-empty) sequence: its history comes from its own state
+        while (t >= seq_end) { ++r; seq_start = cu[r]; seq_end = cu[r + 1]; }
+        load_hist(t);
+      }
+      Vec16<T> o;
 #pragma unroll
-    for (int j = 0; j < W - 1; ++j) {
+      for (int e = 0; e < V; ++e) {
+        win[W - 1][e] = to_f(rows[i].v[e]);
+        float acc = bv[e];
 #pragma unroll
-      for (int e = 0; e < V; ++e) win[j][e] = win[j + 1][e];
+        for (int j = 0; j < W; ++j) acc += wv[j][e] * win[j][e];
+        o.v[e] = from_f<T>(act ? silu<T>(acc) : acc);
+      }
+      st_vec(out + t * out_stride + c0, o);
+#pragma unroll
+      for (int j = 0; j < W - 1; ++j) {
+#pragma unroll
+        for (int e = 0; e < V; ++e) win[j][e] = win[j + 1][e];
+      }
     }
   }
 }
