@@ -83,6 +83,41 @@ __global__ void warp_rownorm_kernel(T* __restrict__ out, const T* __restrict__ x
   }
 }
 
+// The same for rows of 128 in 16 bits, 16-byte aligned: sixteen lanes a row, one load and one store a lane.  Bound by memory:
+// 262144 gated rows are 201 MB; 31 us, 61 with a warp a row and 2-byte accesses.
+template <typename T, int kMode>
+__global__ void __launch_bounds__(256) rownorm_128_kernel(T* __restrict__ out, const T* __restrict__ x, const T* __restrict__ z,
+                                                          const T* __restrict__ w, int64_t rows, float eps) {
+  const int64_t row = (int64_t)blockIdx.x * 16 + (threadIdx.x >> 4);
+  const int l = threadIdx.x & 15;
+  const bool in = row < rows;
+  Vec16<T> a, g, wv;
+  float v[8], ss = 0.f;
+  if (in) {
+    a = ld_vec(x + row * 128 + l * 8);
+    if (kMode >= 2) g = ld_vec(z + row * 128 + l * 8);
+    if (kMode != 1) wv = ld_vec(w + l * 8);
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    v[j] = in ? to_f(a.v[j]) : 0.f;
+    if (kMode == 3 && in) { const float zf = to_f(g.v[j]); v[j] *= zf / (1.f + __expf(-zf)); }
+    ss += v[j] * v[j];
+  }
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if (!in) return;
+  const float inv = (kMode == 1) ? rsqrtf(ss + eps) : rsqrtf(ss / 128 + eps);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    float f = v[j] * inv;
+    if (kMode != 1) f *= to_f(wv.v[j]);
+    if (kMode == 2) { const float zf = to_f(g.v[j]); f *= zf / (1.f + __expf(-zf)); }
+    a.v[j] = from_f<T>(f);
+  }
+  st_vec(out + row * 128 + l * 8, a);
+}
+
 // act: 0 = silu(gate)*up with x = [gate | up]; 1 = gelu_tanh(gate)*up; 2 = swigluoai (interleaved, clamped); 3 = the same
 // function of x = [gate | up] with a given limit
 template <typename T>
@@ -238,6 +273,20 @@ extern "C" int b200_rmsnorm(void* out, const void* x, void* residual, const void
 extern "C" int b200_rownorm(void* out, const void* x, const void* z, const void* w, int64_t rows, int D, float eps,
                             int mode, int dtype, cudaStream_t st) {
   if (rows == 0) return 0;
+  auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  if (D == 128 && dtype != kF32 && aligned(out) && aligned(x) && aligned(z) && aligned(w)) {
+    const int64_t g = (rows + 15) / 16;
+#define B200_ROW128(T)                                                                                                   \
+  switch (mode) {                                                                                                        \
+    case 0: rownorm_128_kernel<T, 0><<<g, 256, 0, st>>>((T*)out, (const T*)x, nullptr, (const T*)w, rows, eps); break;     \
+    case 1: rownorm_128_kernel<T, 1><<<g, 256, 0, st>>>((T*)out, (const T*)x, nullptr, nullptr, rows, eps); break;         \
+    case 2: rownorm_128_kernel<T, 2><<<g, 256, 0, st>>>((T*)out, (const T*)x, (const T*)z, (const T*)w, rows, eps); break; \
+    default: rownorm_128_kernel<T, 3><<<g, 256, 0, st>>>((T*)out, (const T*)x, (const T*)z, (const T*)w, rows, eps); break; \
+  }
+    if (dtype == kBF16) { B200_ROW128(__nv_bfloat16) } else { B200_ROW128(__half) }
+#undef B200_ROW128
+    return (int)cudaGetLastError();
+  }
   int wpb = 8;
   int64_t grid = (rows + wpb - 1) / wpb;
   B200_DISPATCH_DTYPE(dtype, {

@@ -273,6 +273,26 @@ def test_moe_permute_quant(T, k, H, mapped):
     assert bool(((p >= lod[e]) & (p < lod[e + 1])).all())
 
 
+@pytest.mark.parametrize("rows", [1, 15, 16, 333])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("mode", [0, 1, 2, 3])
+def test_row_norms_of_128(rows, dtype, mode):
+    """Rows of 128 in 16-byte pieces against the general kernel (the same rows off a 16-byte boundary): one rounding step apart."""
+    from vllm_kunlun_b200.ops import _ext
+    torch.manual_seed(17)
+    x, z, w = (torch.randn(n, 128, device=DEV).to(dtype) for n in (rows, rows, 1))
+
+    def run(off):
+        def at(t):
+            m = torch.empty(t.numel() + 8, dtype=dtype, device=DEV)[off:off + t.numel()].view(t.shape)
+            return m.copy_(t)
+        out = at(torch.zeros_like(x))
+        _ext.C().rownorm(out, at(x), at(z) if mode >= 2 else None, None if mode == 1 else at(w)[0], 1e-6, mode)
+        return out.float()
+
+    torch.testing.assert_close(run(0), run(1), rtol=2 ** -7 if dtype == torch.bfloat16 else 2 ** -10, atol=1e-6)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("pattern", ["random", "segments"])
 @pytest.mark.parametrize("N,offset,r", [(640, 128, 16), (333, 5, 8), (1030, 0, 12)])
