@@ -293,6 +293,33 @@ def test_row_norms_of_128(rows, dtype, mode):
     torch.testing.assert_close(run(0), run(1), rtol=2 ** -7 if dtype == torch.bfloat16 else 2 ** -10, atol=1e-6)
 
 
+@pytest.mark.parametrize("T,k,E,quant", [(1, 1, 8, True), (16, 8, 128, True), (33, 8, 512, False), (128, 8, 64, True), (300, 3, 16, False)])
+@pytest.mark.parametrize("mapped", [False, True])
+def test_moe_prepare_small_places(T, k, E, quant, mapped):
+    """Places of a small batch's pairs: those of a stable sort by expert, rows and scales the token's."""
+    from vllm_kunlun_b200.ops import _ext
+    torch.manual_seed(18)
+    C, H = _ext.C(), 384
+    x = torch.randn(T, H, device=DEV).bfloat16()
+    ids = torch.rand(T, E, device=DEV).topk(k, -1).indices.int()
+    emap = torch.where(torch.arange(E, device=DEV) % 2 == 0, torch.arange(E, device=DEV) // 2, -1).int() if mapped else None
+    local = E // 2 if mapped else E
+    xs, pos, lod, st = C.moe_prepare_small(x, ids, emap, local, E, quant, None)
+    where = (emap[ids.long()] if mapped else ids).flatten().long()
+    order = torch.sort(torch.where(where < 0, local, where), stable=True).indices
+    want = torch.empty_like(order)
+    want[order] = torch.arange(T * k, device=DEV)
+    assert torch.equal(pos.long(), torch.where(where < 0, -1, want))
+    assert torch.equal(lod.long(), torch.searchsorted(torch.sort(where[where >= 0]).values, torch.arange(local + 1, device=DEV)))
+    pair = (where >= 0).nonzero()[:, 0]
+    p, token = pos[pair].long(), pair // k
+    if quant:
+        want_q, want_s = C.quant_fp8_group(x, False, None, 4)
+        assert torch.equal(xs[p], want_q[token]) and torch.equal(st[:, p], want_s[:, token])
+    else:
+        assert torch.equal(xs[p], x[token])
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("pattern", ["random", "segments"])
 @pytest.mark.parametrize("N,offset,r", [(640, 128, 16), (333, 5, 8), (1030, 0, 12)])
