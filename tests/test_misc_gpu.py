@@ -273,6 +273,34 @@ def test_moe_permute_quant(T, k, H, mapped):
     assert bool(((p >= lod[e]) & (p < lod[e + 1])).all())
 
 
+@pytest.mark.parametrize("T,Hq,Hkv,norm,dtype", [(1, 4, 2, True, torch.bfloat16), (257, 32, 8, False, torch.bfloat16),
+                                                 (300, 5, 2, True, torch.float16), (40, 1, 1, False, torch.float16)])
+@pytest.mark.parametrize("gemma", [False, True])
+def test_qkv_rope_cache_wide_route(T, Hq, Hkv, norm, dtype, gemma):
+    """Heads of 128 in 16-byte pieces against the general kernel, which the same rows take when they start off a 16-byte boundary:
+    sums of 128 squares in another order, so that a value next to a rounding edge may move by one step of the 16-bit type."""
+    from vllm_kunlun_b200.ops import _ext
+    torch.manual_seed(16)
+    C, width = _ext.C(), (Hq + 2 * Hkv) * 128
+    buf = torch.randn(T, width + 8, device=DEV).to(dtype)
+    w = [torch.randn(128, device=DEV).to(dtype) if norm else None for _ in range(2)]
+    pos, slots = torch.randint(-1, 600, (T,), device=DEV), torch.randperm(512, device=DEV)[:T] - 3
+    cos_sin = torch.randn(512, 128, device=DEV)
+    res = []
+    for off in (0, 1):
+        rows = torch.empty(T, width + 8, dtype=dtype, device=DEV)[:, off:off + width]
+        rows.copy_(buf[:, :width])
+        q, cache = torch.zeros(T, Hq * 128, dtype=dtype, device=DEV), torch.zeros(8, 2, Hkv, 64, 128, dtype=dtype, device=DEV)
+        C.qkv_split_norm_rope_cache(q, rows, pos, cos_sin, w[0], w[1], 1e-6, Hq, Hkv, 128, True, gemma, cache, slots)
+        res.append((q.float(), cache.float()))
+    step = 2 ** -7 if dtype == torch.bfloat16 else 2 ** -10
+    for got, want in zip(*res):
+        # two steps: one before the rotation, which mixes two columns, and one behind it
+        torch.testing.assert_close(got, want, rtol=2 * step, atol=4 * step)
+    if not norm:
+        assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
+
+
 @pytest.mark.parametrize("rows", [1, 15, 16, 333])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("mode", [0, 1, 2, 3])
