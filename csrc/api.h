@@ -410,7 +410,7 @@ int b200_paged_attention_generic(void* out, const void* q, const void* kv_cache,
 // ---- gated delta net / conv / MTP glue --------------------------------------------------------
 int b200_causal_conv1d_fwd(void* out, int64_t out_stride, const void* x, int64_t x_stride, const void* w,
                            const void* bias, const int* cu, int R, void* states, const int* slots,
-                           const uint8_t* has_init, int C, int W, int act, int64_t T_, int dtype, cudaStream_t st);
+                           const void* has_init, int init_wide, int C, int W, int act, int64_t T_, int dtype, cudaStream_t st);
 int b200_causal_conv1d_update(void* out, int64_t out_stride, const void* x, int64_t x_stride, void* states,
                               const void* w, const void* bias, const int* slots, const int* has_init, int64_t B, int C,
                               int W, int act, int dtype, cudaStream_t st);
@@ -418,7 +418,7 @@ int b200_gdn_gating(float* g, float* beta, const void* a, int64_t a_stride, cons
                     const float* A_log, const float* dt_bias, int H, int64_t T_, int dtype, cudaStream_t st);
 int b200_gdn_recurrent(void* out, int64_t o_stride, const void* q, const void* k, int64_t qk_stride, const void* v,
                        int64_t v_stride, const float* g, const float* beta, float* states, const int* cu,
-                       const int* slots, const uint8_t* has_init, int R, int Hk, int Hv, int Dk, int Dv, float scale,
+                       const int* slots, const void* has_init, int init_wide, int R, int Hk, int Hv, int Dk, int Dv, float scale,
                        int l2norm, int dtype, int64_t T, int* status, cudaStream_t st);
 // Linear recurrences with a matrix state (linear_attn/recurrence.cu); kind 0 = delta rule with a decay per key channel,
 // 1 = fixed decay per head.  q, k: [T][Hk][Dk], v: [T][H][Dv] column slices of one row-strided tensor.

@@ -1421,13 +1421,19 @@ void rejection_sample(at::Tensor out, const at::Tensor& draft_ids, const at::Ten
         "rejection_sample");
 }
 
+// 1 for 32-bit flags, 0 for bytes
+int flag_width(const at::Tensor& flags) {
+  TORCH_CHECK(flags.is_contiguous() && (flags.scalar_type() == at::kInt || flags.element_size() == 1));
+  return flags.scalar_type() == at::kInt;
+}
+
 void causal_conv1d_fwd(at::Tensor out, const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& bias,
                        const at::Tensor& cu, at::Tensor states, const at::Tensor& slots, const at::Tensor& has_init,
                        bool act) {
   TORCH_CHECK(x.dim() == 2 && x.stride(1) == 1 && out.stride(1) == 1 && w.is_contiguous() && states.is_contiguous());
   check(b200_causal_conv1d_fwd(out.data_ptr(), out.stride(0), x.data_ptr(), x.stride(0), w.data_ptr(), opt_ptr(bias),
                                cu.data_ptr<int>(), (int)slots.size(0), states.data_ptr(), slots.data_ptr<int>(),
-                               (const uint8_t*)has_init.data_ptr(), (int)x.size(1), (int)w.size(1), act, x.size(0),
+                               has_init.data_ptr(), flag_width(has_init), (int)x.size(1), (int)w.size(1), act, x.size(0),
                                dtype_code(x), stream()), "causal_conv1d_fwd", 2);
 }
 
@@ -1467,7 +1473,7 @@ void gdn_recurrent(at::Tensor out, const at::Tensor& q, const at::Tensor& k, con
   }
   check(b200_gdn_recurrent(out.data_ptr(), out.stride(0), q.data_ptr(), k.data_ptr(), q.stride(0), v.data_ptr(), v.stride(0),
                            g.data_ptr<float>(), beta.data_ptr<float>(), states.data_ptr<float>(), cu.data_ptr<int>(),
-                           slots.data_ptr<int>(), (const uint8_t*)has_init.data_ptr(), (int)slots.size(0), (int)q.size(1),
+                           slots.data_ptr<int>(), has_init.data_ptr(), flag_width(has_init), (int)slots.size(0), (int)q.size(1),
                            (int)v.size(1), (int)q.size(2), (int)v.size(2), (float)scale, l2norm, dtype_code(q), q.size(0),
                            gs.status.data_ptr<int>(), stream()),
         "gdn_recurrent");

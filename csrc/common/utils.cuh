@@ -24,6 +24,15 @@ __device__ __forceinline__ float pow2_ceil(float x) {
   return __uint_as_float((__float_as_uint(x) + 0x7fffffu) & 0xff800000u);
 }
 
+// One flag per request, in bytes or in 32-bit integers: callers hold either, and a conversion would be a launch of its own.
+struct InitFlags {
+  const void* p;
+  int wide;
+  __device__ __forceinline__ bool operator[](int r) const {
+    return wide ? static_cast<const int*>(p)[r] != 0 : static_cast<const uint8_t*>(p)[r] != 0;
+  }
+};
+
 // 16-byte vector of T
 template <typename T>
 struct alignas(16) Vec16 {

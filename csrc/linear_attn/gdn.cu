@@ -15,7 +15,7 @@
 namespace b200 {
 // gdn_chunk.cu
 int gdn_chunk(void* out, int64_t o_stride, const void* q, const void* k, int64_t qk_stride, const void* v, int64_t v_stride,
-              const float* g, const float* beta, float* states, const int* cu, const int* slots, const uint8_t* has_init,
+              const float* g, const float* beta, float* states, const int* cu, const int* slots, InitFlags has_init,
               int64_t T, int R, int Hk, int Hv, float scale, int min_len, int* status, cudaStream_t st);
 
 namespace {
@@ -45,7 +45,7 @@ template <typename T, int W>
 __global__ void __launch_bounds__(128) conv1d_fwd_kernel(T* __restrict__ out, int64_t out_stride, const T* __restrict__ x,
                                                          int64_t x_stride, const T* __restrict__ w, const T* __restrict__ bias,
                                                          const int* __restrict__ cu, int R, const T* __restrict__ states,
-                                                         const int* __restrict__ slots, const uint8_t* __restrict__ has_init,
+                                                         const int* __restrict__ slots, InitFlags has_init,
                                                          int C, int act, int64_t Ttot) {
   constexpr int V = Vec16<T>::N;
   const int c0 = (blockIdx.x * blockDim.x + threadIdx.x) * V;
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(128) conv1d_fwd_kernel(T* __restrict__ out, in
   auto load_hist = [&](int64_t t) {  // fill win[0 .. W-2] with the W-1 rows in front of token t
     const int p = (int)t - seq_start;
     const int slot = slots[r];
-    const bool init = has_init[r] != 0 && slot >= 0;
+    const bool init = has_init[r] && slot >= 0;
 #pragma unroll
     for (int j = 0; j < W - 1; ++j) {
       const int q = p - (W - 1) + j;
@@ -129,13 +129,13 @@ template <typename T>
 __global__ void conv1d_fwd_generic_kernel(T* __restrict__ out, int64_t out_stride, const T* __restrict__ x, int64_t x_stride,
                                           const T* __restrict__ w, const T* __restrict__ bias, const int* __restrict__ cu,
                                           int R, const T* __restrict__ states, const int* __restrict__ slots,
-                                          const uint8_t* __restrict__ has_init, int C, int W, int act, int64_t Ttot) {
+                                          InitFlags has_init, int C, int W, int act, int64_t Ttot) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t t = blockIdx.y;
   if (c >= C || t >= Ttot) return;
   const int r = find_seq(cu, R, (int)t);
   const int p = (int)t - cu[r], slot = slots[r];
-  const bool init = has_init[r] != 0 && slot >= 0;
+  const bool init = has_init[r] && slot >= 0;
   float acc = bias ? to_f(bias[c]) : 0.f;
   for (int j = 0; j < W; ++j) {
     const int q = p - (W - 1) + j;
@@ -152,13 +152,13 @@ __global__ void conv1d_fwd_generic_kernel(T* __restrict__ out, int64_t out_strid
 template <typename T>
 __global__ void conv1d_state_kernel(T* __restrict__ states, const T* __restrict__ x, int64_t x_stride,
                                     const int* __restrict__ cu, const int* __restrict__ slots,
-                                    const uint8_t* __restrict__ has_init, int C, int W) {
+                                    InitFlags has_init, int C, int W) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const int r = blockIdx.y;
   if (c >= C) return;
   const int s = cu[r], L = cu[r + 1] - s, slot = slots[r];
   if (L == 0 || slot < 0) return;
-  const bool init = has_init[r] != 0;
+  const bool init = has_init[r];
   T* st = states + (int64_t)slot * (W - 1) * C + c;
   for (int j = 0; j < W - 1; ++j) {
     const int q = L - (W - 1) + j;
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(128) gdn_recurrent_kernel(
     T* __restrict__ out, int64_t o_stride, const T* __restrict__ q, const T* __restrict__ k, int64_t qk_stride,
     const T* __restrict__ v, int64_t v_stride, const float* __restrict__ g, const float* __restrict__ beta,
     float* __restrict__ states /*[slots, Hv, Dv, DK]*/, const int* __restrict__ cu, const int* __restrict__ slots,
-    const uint8_t* __restrict__ has_init, int Hk, int Hv, int Dv, float scale, int l2norm, int chunk_min) {
+    InitFlags has_init, int Hk, int Hv, int Dv, float scale, int l2norm, int chunk_min) {
   static_assert(DK % 16 == 0 && DK <= 128, "DK");
   constexpr int QW = DK / 4;                      // state columns per thread
   constexpr int CH = kGdnChunk;
@@ -369,14 +369,14 @@ __global__ void __launch_bounds__(128) gdn_step_kernel(
     T* __restrict__ out, int64_t o_stride, const T* __restrict__ q, const T* __restrict__ k, int64_t qk_stride,
     const T* __restrict__ v, int64_t v_stride, const float* __restrict__ g, const float* __restrict__ beta,
     float* __restrict__ states /*[slots, Hv, Dv, 128]*/, const int* __restrict__ cu, const int* __restrict__ slots,
-    const uint8_t* __restrict__ has_init, int Hk, int Hv, int Dv, float scale, int l2norm) {
+    InitFlags has_init, int Hk, int Hv, int Dv, float scale, int l2norm) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int hv = blockIdx.y, r = blockIdx.z, hk = hv / (Hv / Hk), row0 = blockIdx.x * 32 + warp * 8;
   const int s = cu[r], L = cu[r + 1] - s, slot = slots[r];
   if (L == 0 || slot < 0) return;
   float4* sp = reinterpret_cast<float4*>(states + (((int64_t)slot * Hv + hv) * Dv + row0) * 128) + lane;
   float4 S[8];
-  const bool init = has_init[r] != 0;
+  const bool init = has_init[r];
 #pragma unroll
   for (int i = 0; i < 8; ++i) S[i] = init ? sp[i * 32] : make_float4(0.f, 0.f, 0.f, 0.f);
   for (int t = s; t < s + L; ++t) {
@@ -451,7 +451,7 @@ namespace b200 {
 namespace {
 template <typename T>
 int launch_conv_fwd(void* out, int64_t out_stride, const void* x, int64_t x_stride, const void* w, const void* bias,
-                    const int* cu, int R, void* states, const int* slots, const uint8_t* has_init, int C, int W, int act,
+                    const int* cu, int R, void* states, const int* slots, InitFlags has_init, int C, int W, int act,
                     int64_t T_, cudaStream_t st) {
   constexpr int V = Vec16<T>::N;
   if (C % V != 0 || (x_stride % V) != 0 || (out_stride % V) != 0) return 3;
@@ -484,11 +484,11 @@ int launch_conv_fwd(void* out, int64_t out_stride, const void* x, int64_t x_stri
 
 extern "C" int b200_causal_conv1d_fwd(void* out, int64_t out_stride, const void* x, int64_t x_stride, const void* w,
                                       const void* bias, const int* cu, int R, void* states, const int* slots,
-                                      const uint8_t* has_init, int C, int W, int act, int64_t T_, int dtype, cudaStream_t st) {
+                                      const void* has_init, int init_wide, int C, int W, int act, int64_t T_, int dtype, cudaStream_t st) {
   if (W < 1) return 3;
   if (T_ == 0) return 0;
   B200_DISPATCH_DTYPE(dtype, return (b200::launch_conv_fwd<T>(out, out_stride, x, x_stride, w, bias, cu, R, states, slots,
-                                                              has_init, C, W, act, T_, st)));
+                                                              b200::InitFlags{has_init, init_wide}, C, W, act, T_, st)));
   return 1;
 }
 
@@ -515,10 +515,11 @@ extern "C" int b200_gdn_gating(float* g, float* beta, const void* a, int64_t a_s
 
 extern "C" int b200_gdn_recurrent(void* out, int64_t o_stride, const void* q, const void* k, int64_t qk_stride, const void* v,
                                   int64_t v_stride, const float* g, const float* beta, float* states, const int* cu,
-                                  const int* slots, const uint8_t* has_init, int R, int Hk, int Hv, int Dk, int Dv, float scale,
+                                  const int* slots, const void* has_init, int init_wide, int R, int Hk, int Hv, int Dk, int Dv, float scale,
                                   int l2norm, int dtype, int64_t T_, int* status, cudaStream_t st) {
   if (R == 0) return 0;
   if (Dv % 32 != 0 || Hv % Hk != 0) return 3;
+  const b200::InitFlags flags{has_init, init_wide};
   // Prompts go through the chunked form (4 x 2048 tokens, 32 heads: 3308 us as a scan, 221 us).  Normalised q and k only: the
   // inverse that it needs is of a matrix whose entries the norms bound.  T_ - (R - 1) rows are the most that one request can have
   // when each of the others has a row: decode steps go straight to the scan.
@@ -526,7 +527,7 @@ extern "C" int b200_gdn_recurrent(void* out, int64_t o_stride, const void* q, co
   int chunk_min = INT_MAX;
   if (dtype == b200::kBF16 && l2norm && Dk == 128 && Dv == 128 && T_ - (R - 1) >= min_len) {
     chunk_min = R == 1 ? 1 : min_len;   // a lone request needs no second launch
-    const int rc = b200::gdn_chunk(out, o_stride, q, k, qk_stride, v, v_stride, g, beta, states, cu, slots, has_init, T_, R, Hk,
+    const int rc = b200::gdn_chunk(out, o_stride, q, k, qk_stride, v, v_stride, g, beta, states, cu, slots, flags, T_, R, Hk,
                                    Hv, scale, chunk_min, status, st);
     if (rc > 0) return rc;
     if (rc == 0 && R == 1) return 0;
@@ -539,13 +540,13 @@ extern "C" int b200_gdn_recurrent(void* out, int64_t o_stride, const void* q, co
   if (Dk == 128 && T_ <= 2 * (int64_t)R && chunk_min == INT_MAX && qk_stride % 4 == 0 && aligned(q) && aligned(k)) {
     B200_DISPATCH_DTYPE(dtype, (b200::gdn_step_kernel<T><<<grid, 128, 0, st>>>(
                                    (T*)out, o_stride, (const T*)q, (const T*)k, qk_stride, (const T*)v, v_stride, g, beta,
-                                   states, cu, slots, has_init, Hk, Hv, Dv, scale, l2norm)));
+                                   states, cu, slots, flags, Hk, Hv, Dv, scale, l2norm)));
     return cudaGetLastError() != cudaSuccess;
   }
 #define B200_GDN_LAUNCH(DK)                                                                                          \
   B200_DISPATCH_DTYPE(dtype, (b200::gdn_recurrent_kernel<T, DK><<<grid, 128, 0, st>>>(                                  \
                                  (T*)out, o_stride, (const T*)q, (const T*)k, qk_stride, (const T*)v, v_stride, g, beta, \
-                                 states, cu, slots, has_init, Hk, Hv, Dv, scale, l2norm, chunk_min)))
+                                 states, cu, slots, flags, Hk, Hv, Dv, scale, l2norm, chunk_min)))
   if (Dk == 128) { B200_GDN_LAUNCH(128); }
   else if (Dk == 64) { B200_GDN_LAUNCH(64); }
   else if (Dk == 32) { B200_GDN_LAUNCH(32); }

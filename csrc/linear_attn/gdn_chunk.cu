@@ -74,7 +74,7 @@ struct Params {
   const float *g, *beta;
   float* states;
   const int *cu, *slots;
-  const uint8_t* has_init;
+  InitFlags has_init;
   int* status;
   int64_t o_stride;
   int Hk, Hv, min_len;
@@ -616,7 +616,7 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(const __grid_con
 // Requests of at least `min_len` of the T tokens; the others are left as they are.  Dk = Dv = 128, bf16, L2-normalised q and
 // k.  Returns -1, with nothing launched, when q, k or v cannot be read by tensor maps (alignment, strides).
 int gdn_chunk(void* out, int64_t o_stride, const void* q, const void* k, int64_t qk_stride, const void* v, int64_t v_stride,
-              const float* g, const float* beta, float* states, const int* cu, const int* slots, const uint8_t* has_init,
+              const float* g, const float* beta, float* states, const int* cu, const int* slots, InitFlags has_init,
               int64_t T, int R, int Hk, int Hv, float scale, int min_len, int* status, cudaStream_t st) {
   CUtensorMap tm[3];
   if (T > INT_MAX || R > 65535 || qk_stride < Hk * 128 || v_stride < Hv * 128) return -1;

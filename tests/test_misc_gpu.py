@@ -202,6 +202,30 @@ def test_gated_delta_rule_steps(lens, Hk, Hv, Dv, dtype, l2norm):
     torch.testing.assert_close(got, want, atol=1e-5, rtol={torch.float32: 1e-4, torch.float16: 2 ** -9, torch.bfloat16: 2 ** -7}[dtype])
 
 
+@pytest.mark.parametrize("flags", [torch.int32, torch.bool, torch.uint8, torch.int64])
+@pytest.mark.parametrize("W", [2, 4, 9])
+def test_single_token_convolution_and_flags(flags, W):
+    """Per-request flags of every type that callers have, as the convolutions read them."""
+    torch.manual_seed(19)
+    R, ch = 5, 264
+    x, w = torch.randn(R, ch).bfloat16(), torch.randn(ch, W).bfloat16()
+    base = torch.randn(R + 1, W - 1, ch).bfloat16()
+    slots, init = torch.tensor([3, 0, 4, 5, 1], dtype=torch.int32), torch.tensor([1, 0, 1, 1, 0]).to(flags)
+    cu = torch.arange(R + 1, dtype=torch.int32)
+    for one in (True, False):
+        res = []
+        for dev in (DEV, "cpu"):
+            st = base.clone().to(dev)
+            if one:
+                o = ops.causal_conv1d_update(x.to(dev), st, w.to(dev), None, slots.to(dev), True, init.to(dev))
+            else:
+                o = ops.causal_conv1d_fn(x.to(dev), w.to(dev), None, cu.to(dev), st, slots.to(dev), init.to(dev), True)
+            res.append((o.cpu().float(), st.cpu()))
+        # fp32 sums of at most nine products, rounded to bf16 once: one step
+        torch.testing.assert_close(res[0][0], res[1][0], rtol=2 ** -7, atol=1e-5)
+        assert torch.equal(res[0][1], res[1][1])
+
+
 @pytest.mark.parametrize("rows", [[300, 0, 1, 63, 64, 65], [127, 128, 129, 257]])
 @pytest.mark.parametrize("N,K,bias", [(512, 256, False), (384, 128, True), (200, 384, False)])
 def test_grouped_fp8_wide_tiles(rows, N, K, bias):

@@ -616,11 +616,16 @@ def rejection_sample(draft_token_ids, num_draft, target_probs, bonus_token_ids, 
 
 # ----------------------------------------------------------------------------- conv / gated delta net
 
+def _flags(t):
+    """Per-request flags as the kernels read them: 32-bit integers and bytes as they are, others converted."""
+    return t.contiguous() if t.dtype in (torch.int32, torch.uint8, torch.bool) else t.to(torch.uint8).contiguous()
+
+
 def causal_conv1d_fn(x, weight, bias, cu_seqlens, conv_states, state_indices, has_initial_state, activation=True):
     if x.is_cuda:
         out = torch.empty(x.shape, dtype=x.dtype, device=x.device)
         _c().causal_conv1d_fwd(out, x, weight, bias, cu_seqlens.int(), conv_states, state_indices.int(),
-                               has_initial_state.to(torch.uint8), activation)
+                               _flags(has_initial_state), activation)
         return out
     return _rx.causal_conv1d_fn(x, weight, bias, cu_seqlens, conv_states, state_indices, has_initial_state, activation)
 
@@ -675,7 +680,7 @@ def gated_delta_rule(q, k, v, g, beta, states, cu_seqlens, state_indices, has_in
     if len(long_rows) < len(cu_seqlens) - 1:
         if q.is_cuda:
             _c().gdn_recurrent(out, q, k, v, g, beta, states, cu_seqlens.int(), slots.int(),
-                               has_initial_state.to(torch.uint8), scale, use_qk_l2norm)
+                               _flags(has_initial_state), scale, use_qk_l2norm)
         else:
             for r in range(len(cu_seqlens) - 1):
                 s, e = int(cu_seqlens[r]), int(cu_seqlens[r + 1])
