@@ -58,7 +58,7 @@ struct Smem {
   float m[32][32];
   Scalars sc[2];
   float ones[8];
-  uint64_t raw[2], full[2], d0, d0_read, t_ready, s_ready, x1, x2, r_ready, u_full, ut_ready, uo_ready, d3, y, o_read, end;
+  uint64_t raw[2], full[2], d0, d0_read, t_ready, s_ready, x1, x2, r_ready, u_full, ut_ready, uo_ready, d3, y[2], o_read, end;   // y: one per buffer of P
   uint32_t tmem;
   int abort_flag;
 };
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(const __grid_con
     for (int i = 0; i < 8; ++i) sm.ones[i] = 1.f;
     for (int i = 0; i < 2; ++i) { mbar_init(&sm.raw[i], 1); mbar_init(&sm.full[i], 64); }
     mbar_init(&sm.d0, 1); mbar_init(&sm.x1, 1); mbar_init(&sm.x2, 1); mbar_init(&sm.u_full, 1);
-    mbar_init(&sm.d3, 1); mbar_init(&sm.y, 1); mbar_init(&sm.end, 1);
+    mbar_init(&sm.d3, 1); mbar_init(&sm.y[0], 1); mbar_init(&sm.y[1], 1); mbar_init(&sm.end, 1);
     mbar_init(&sm.d0_read, 4); mbar_init(&sm.t_ready, kPrep);
     mbar_init(&sm.s_ready, 8); mbar_init(&sm.r_ready, 8); mbar_init(&sm.ut_ready, 8); mbar_init(&sm.uo_ready, 8);
     mbar_init(&sm.o_read, 8);
@@ -257,7 +257,9 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(const __grid_con
       const int row = (warp & 1) * 32 + lane;
       const uint32_t td = tm + kD0 + ((uint32_t)(warp * 32) << 16);
       const float gh = sc.gh[row], gl = sc.gl[row], fac = is_q ? sc.rq[row] : sc.beta[row] * sc.rk[row];
-      if (is_q && n >= 2) wait(&sm.y, n - 2, 903);  // the output of chunk n - 2 has been computed from this buffer of P
+      // The output of chunk n - 2 has been computed from this buffer of P.  A barrier per buffer: its next phase needs the P that is
+      // written here, so it cannot complete before this wait has looked (the output of chunk n - 1, in the other buffer, can).
+      if (is_q && n >= 2) wait(&sm.y[n & 1], (n - 2) >> 1, 903);
       const int last = is_q ? row : row - 1;           // last column that is kept
       // what lies above the diagonal of a warp's 32 rows is zero and was set at the start
 #pragma unroll 1
@@ -350,7 +352,7 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(const __grid_con
       tc_fence_after_sync();
     };
     auto write_out = [&](int c) {                      // outputs of chunk c, this thread: one dv, 32 tokens
-      wait_tc(&sm.y, c, 910);
+      wait_tc(&sm.y[c & 1], c >> 1, 910);
       uint32_t o[32];
       tmem_ld_x32(tl + kX2 + wg * 32, o);
       tmem_ld_wait();
@@ -477,7 +479,7 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(const __grid_con
           sc.gh[2 * lane + 1] = (float)sum;
           sc.gl[2 * lane + 1] = (float)(sum - (double)(float)sum);
         }
-        wait(&sm.raw[st], c >> 1, 905);
+        wait(&sm.raw[st], c >> 1, 906);
         // a thread = one row of K, Q and V.  Rows behind the request's end are another request's: zeros instead
         uint64_t k2[2] = {0, 0}, q2[2] = {0, 0};
         if (lt >= n) {
@@ -595,7 +597,7 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(const __grid_con
       wait_one(&sm.uo_ready, c, 927);
       tc_fence_after_sync();
       tokens_times(kX2, kUo, p_addr + (c & 1) * 3 * kPiece, 1);
-      umma_commit(&sm.y);
+      umma_commit(&sm.y[c & 1]);
     }
     umma_commit(&sm.end);
     for (uint32_t i = 0; i < (1u << 16); ++i)          // nothing is in flight when TMEM is given back (bounded)

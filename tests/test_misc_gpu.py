@@ -179,6 +179,27 @@ def test_gated_delta_rule_chunk_edges(lens, Hk, Hv, offset):
     torch.testing.assert_close(got[:n].float(), want[:n].float(), atol=1e-3, rtol=2 ** -7)
 
 
+@pytest.mark.parametrize("lens", [[4096], [2048, 1000, 3000]])
+def test_gated_delta_rule_many_chunks(lens):
+    """Up to 64 chunks a request: no wait gives up, and the results are the oracle's within the bounds given above."""
+    from vllm_kunlun_b200.ops.gemm_cuda import check_status
+    torch.manual_seed(21)
+    T, R, Hk, Hv = sum(lens), len(lens), 1, 2
+    q, k, v = (torch.randn(T, h, 128).bfloat16() for h in (Hk, Hk, Hv))
+    g, beta = -torch.rand(T, Hv) * 0.05, torch.rand(T, Hv)
+    slots, init = torch.arange(R).int(), torch.zeros(R).int()
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32)
+
+    def run(dev):
+        st = torch.zeros(R, Hv, 128, 128, device=dev)
+        return ops.gated_delta_rule(*(t.to(dev) for t in (q, k, v, g, beta)), st, cu.to(dev), slots.to(dev), init.to(dev)).cpu(), st.cpu()
+
+    (got, got_st), (want, want_st) = run(DEV), run("cpu")
+    check_status()
+    torch.testing.assert_close(got_st, want_st, atol=1e-4, rtol=1e-4)
+    torch.testing.assert_close(got.float(), want.float(), atol=1e-3, rtol=2 ** -7)
+
+
 @pytest.mark.parametrize("lens,Hk,Hv,Dv,dtype", [([1] * 5, 2, 4, 128, torch.bfloat16), ([2, 0, 1, 3], 1, 2, 64, torch.float16),
                                                  ([1, 1, 2], 2, 2, 32, torch.float32)])
 @pytest.mark.parametrize("l2norm", [True, False])
