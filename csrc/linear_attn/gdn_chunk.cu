@@ -13,12 +13,15 @@
 // pairs of floats (from doubles), because a difference of two sums is what is raised to a power.
 //
 // Warps 0-3: A, T and P of the chunk ahead; warps 4-11: the chain S -> R -> U -> S, a thread = one row x half of the
-// columns, S in registers; warp 12: MMA issue; warps 13, 14: loads, norms and gates, up to two chunks ahead.  What bounds it is that chain: three dependent products
+// columns, S in registers; warp 12: MMA issue; warps 13 to 15: loads, norms and gates, up to two chunks ahead.  What bounds it is that chain: three dependent products
 // (24, 24 and 12 MMA steps) with a pass through registers between them, 64 tokens a turn; the outputs and the
 // next chunk's T are computed beside it.  6 us a chunk and CTA, of which 2.9 are products (4 x 2048 tokens, 32 heads:
 // 217 us, 3308 us as a scan; 1 x 4096 tokens, 16 heads: 393 us, 1910 us as a scan).  Waits and loops are kept small (70 KB of
 // code in all): unrolled throughout, the roles evicted one another's instructions and a chunk took 13 us.  Every wait is bounded; a CTA that gives up sets the status word and runs out.
-// Zeros hide the keys behind a query, so a NaN or an infinity in a token reaches the whole chunk of its own request.
+// Zeros hide later keys, and zero times a NaN or an infinity is not zero: a chunk ends in front of a token with such a value in k,
+// v, its gate or beta, which is the first token of the next one.  So it reaches its own and later tokens only, as in the scan
+// (one in q stays in its own row of every product).  Looking for them costs 8 of 214 us (4 x 2048 tokens): the loads are on
+// the way to the next chunk's T.  Finite inputs whose squares or products overflow are taken for such values or not found.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <limits.h>
@@ -45,7 +48,8 @@ constexpr int kPitch = 68;                      // floats of a row of the fp32 6
 struct Scalars {                                // per token of a chunk
   float beta[kC], gh[kC], gl[kC], rk[kC], rq[kC];   // gate sums in log2 units, high and low part; inverse norms (rq with scale)
   float c1[kC], c2[kC], c3[kC];                 // beta exp(c) rk;  exp(c_63 - c) rk;  exp(c) rq
-  float decay, pad[3];                          // exp(c_63)
+  float decay;                                  // exp(c_63)
+  int n, pad[2];                                // tokens of the chunk
 };
 
 struct Smem {
@@ -61,6 +65,8 @@ struct Smem {
   uint64_t raw[2], full[2], d0, d0_read, t_ready, s_ready, x1, x2, r_ready, u_full, ut_ready, uo_ready, d3, y[2], o_read, end;   // y: one per buffer of P
   uint32_t tmem;
   int abort_flag;
+  int cut;                                      // tokens of a chunk that ends in front of a value that is not finite
+  int n_prep;                                   // tokens of the chunk, one copy for the four warps of the first role
 };
 constexpr int kSmemBytes = (int)sizeof(Smem) + 1024;
 static_assert(kSmemBytes <= 227 * 1024, "shared memory");
@@ -114,6 +120,12 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// acc + 0 * v on pairs of bf16: acc stays zero while everything is finite, and is a NaN from then on
+__device__ __forceinline__ uint32_t times_zero(uint32_t v, uint32_t acc) {
+  uint32_t d;
+  asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(v), "r"(0u), "r"(acc));
+  return d;
+}
 // squares of two bf16 in fp32 added to a pair
 __device__ __forceinline__ uint64_t square2(uint32_t v, uint64_t acc) {
   const uint64_t x = f2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
@@ -148,6 +160,20 @@ __device__ __forceinline__ void store_pieces_smem(uint8_t* base, int row, int c,
   *reinterpret_cast<uint4*>(base + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
   *reinterpret_cast<uint4*>(base + kPiece + off) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
   *reinterpret_cast<uint4*>(base + 2 * kPiece + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+}
+// Tokens of a chunk that its loader has published; `left` of the request are not in a chunk yet.  At least one and none too many
+// whatever was read (after a wait that gave up): every role ends, and writes stay within the request.
+__device__ __forceinline__ int take_chunk(int n, int& left) {
+  n = min(max(n, 1), min(kC, left));
+  left -= n;
+  return n;
+}
+// a barrier of n threads that tells all of them whether `any` holds for one
+__device__ __forceinline__ bool bar_any(int id, int n, bool any) {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred q, p;\n\tsetp.ne.u32 q, %3, 0;\n\tbar.red.or.pred p, %1, %2, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(r) : "r"(id), "r"(n), "r"((uint32_t)any) : "memory");
+  return r != 0;
 }
 __device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 
@@ -201,7 +227,6 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(const __grid_con
   const int hv = blockIdx.x, r = blockIdx.y;
   const int s0 = p.cu[r], L = p.cu[r + 1] - s0, slot = p.slots[r];
   if (L < p.min_len || slot < 0) return;
-  const int n_chunks = (L + kC - 1) / kC;
   extern __shared__ uint8_t smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -249,9 +274,11 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(const __grid_con
     // ------------------------------------------------------------------ the chunk ahead: A, T, P
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsPrep));
     const bool is_q = warp >= 2;                 // warps 2, 3: P (lanes 64-127 of D0); 0, 1: A
-    for (int n = 0; n < n_chunks; ++n) {
+    int left = L;
+    for (int n = 0;; ++n) {
       const Scalars& sc = sm.sc[n & 1];
       wait(&sm.full[n & 1], n >> 1, 901);
+      if (tid == 0) sm.n_prep = sc.n;
       wait(&sm.d0, n, 902);
       tc_fence_after_sync();
       const int row = (warp & 1) * 32 + lane;
@@ -312,6 +339,7 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(const __grid_con
         for (int i = 0; i < 8; ++i) sm.f[b0 + i][b0 + col] = t[i];
       }
       bar_sync(2, kPrep);
+      take_chunk(sm.n_prep, left);                     // the same for all four: they meet at barriers, after a failure too
       join_blocks<8>(sm, warp, lane);
       join_blocks<16>(sm, warp, lane);
       join_blocks<32>(sm, warp, lane);
@@ -326,6 +354,7 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(const __grid_con
       fence_proxy_async_smem();
       mbar_arrive(&sm.t_ready);
       bar_sync(2, kPrep);                              // sm.f and sm.a are written again for the next chunk
+      if (left == 0) break;
     }
   } else if (warp < 12) {
     // ------------------------------------------------------------------ the chain
@@ -351,30 +380,33 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(const __grid_con
       wait(bar, phase, code);
       tc_fence_after_sync();
     };
-    auto write_out = [&](int c) {                      // outputs of chunk c, this thread: one dv, 32 tokens
+    int n = 0, left = L;                               // tokens of the chunk; of the request behind it
+    __nv_bfloat16* dst = p.out + (s0 + wg * 32) * p.o_stride + hv * 128 + dv;
+    auto write_out = [&](int c, int tokens) {          // outputs of chunk c, this thread: one dv, 32 tokens
       wait_tc(&sm.y[c & 1], c >> 1, 910);
       uint32_t o[32];
       tmem_ld_x32(tl + kX2 + wg * 32, o);
       tmem_ld_wait();
       arrive(&sm.o_read);
-      const int t0 = c * kC + wg * 32;
-      __nv_bfloat16* dst = p.out + (s0 + (int64_t)t0) * p.o_stride + hv * 128 + dv;
+      __nv_bfloat16* at = dst;
 #pragma unroll
-      for (int j = 0; j < 32; ++j, dst += p.o_stride)
-        if (t0 + j < L) *dst = __float2bfloat16(__uint_as_float(o[j]));
+      for (int j = 0; j < 32; ++j, at += p.o_stride)
+        if (wg * 32 + j < tokens) *at = __float2bfloat16(__uint_as_float(o[j]));
+      dst += tokens * p.o_stride;
     };
     for (int c = 0;; ++c) {
       const int st = c & 1;
       const Scalars& sc = sm.sc[st];
-      if (c < n_chunks) {
+      if (left > 0) {
         wait_tc(&sm.d0_read, c, 911);                  // D0 lies over the pieces of S
         store_pieces(tl + kSp + wg * 32, 64, S);
         store_pieces(tl + kSp + wg * 32 + 16, 64, S + 32);
         arrive(&sm.s_ready);
       }
-      if (c > 0) write_out(c - 1);
-      if (c == n_chunks) break;
+      if (c > 0) write_out(c - 1, n);
+      if (left == 0) break;
       wait(&sm.full[st], c >> 1, 912);
+      n = take_chunk(__shfl_sync(0xffffffffu, sc.n, 0), left);   // one value for the warp, after a failure too
       wait_tc(&sm.x1, c, 913);
       uint32_t x[32];
       float w[32];
@@ -438,20 +470,23 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(const __grid_con
   } else {
     // ------------------------------------------------------------------ MMA issue, loads
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
-    if (warp == 13 || warp == 14) {
-      // ------------------------------------------------------------------ loads, norms and gates (warps 13 and 14)
-      const int lt = tid - 13 * 32;              // 0 .. 63
+    if (warp >= 13) {
+      // ------------------------------------------------------------------ loads, norms and gates (13, 14), what is not finite in v (15)
+      const int lt = tid - 13 * 32;              // 0 .. 63, a token of the chunk
       const int hk = hv / (p.Hv / p.Hk);
       int issued = 0;
-      for (int c = 0; c < n_chunks; ++c) {
-        const int st = c & 1, n = L - c * kC;
-        const int64_t tok0 = s0 + (int64_t)c * kC;
+      for (int c = 0, pos = 0; pos < L; ++c) {
+        const int st = c & 1;
+        const int64_t tok0 = s0 + (int64_t)pos;
         Scalars& sc = sm.sc[st];
-        const float beta = lt < n ? p.beta[(tok0 + lt) * p.Hv + hv] : 0.f;
+        int n = min(kC, L - pos);
+        float beta = lt < n ? p.beta[(tok0 + lt) * p.Hv + hv] : 0.f;
+        bool bad = !(fabsf(beta) < INFINITY) && lt > 0;   // a value that is not finite behind the chunk's first token
         double first = 0., sum = 0.;             // gate sums up to tokens 2 lane and 2 lane + 1 (warp 13)
         if (warp == 13) {
           const float g0 = 2 * lane < n ? p.g[(tok0 + 2 * lane) * p.Hv + hv] : 0.f;
           const float g1 = 2 * lane + 1 < n ? p.g[(tok0 + 2 * lane + 1) * p.Hv + hv] : 0.f;
+          bad |= (!(g0 < INFINITY) && lane > 0) || !(g1 < INFINITY);
           // a gate below -128 is a factor of zero in fp32 either way; clamped, the sums stay finite (a NaN stays one)
           const double a = (g0 < -128.f ? -128.f : g0) * 1.4426950408889634, b = (g1 < -128.f ? -128.f : g1) * 1.4426950408889634;
           sum = a + b;
@@ -460,7 +495,8 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(const __grid_con
             const double up = __shfl_up_sync(0xffffffffu, sum, o);
             if (lane >= o) sum += up;
           }
-          first = sum - b;
+          first = __shfl_up_sync(0xffffffffu, sum, 1);   // not sum - b: b may be a NaN
+          first = lane == 0 ? a : first + a;
         }
         if (c >= 2) wait(&sm.d3, c - 2, 904);    // the last reader of this stage
         if (lt == 0 && !failed) {
@@ -480,9 +516,59 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(const __grid_con
           sc.gl[2 * lane + 1] = (float)(sum - (double)(float)sum);
         }
         wait(&sm.raw[st], c >> 1, 906);
-        // a thread = one row of K, Q and V.  Rows behind the request's end are another request's: zeros instead
-        uint64_t k2[2] = {0, 0}, q2[2] = {0, 0};
-        if (lt >= n) {
+        float k2 = 0.f, q2 = 0.f;
+        if (warp == 15) {                        // (rows behind the request's end, too: they are told apart below)
+          uint32_t acc[4] = {0, 0, 0, 0};
+#pragma unroll 8
+          for (int i = 0; i < 32; ++i) {
+            const uint4 a = *reinterpret_cast<const uint4*>(sm.v[st] + i * 512 + lane * 16);
+            acc[0] = times_zero(a.x, acc[0]);
+            acc[1] = times_zero(a.y, acc[1]);
+            acc[2] = times_zero(a.z, acc[2]);
+            acc[3] = times_zero(a.w, acc[3]);
+          }
+          bad = ((acc[0] | acc[1] | acc[2] | acc[3]) & 0x7fff7fffu) != 0;
+        } else if (lt < n) {                     // a thread = one row of K and Q
+          uint64_t k4[2] = {0, 0}, q4[2] = {0, 0};
+#pragma unroll 4
+          for (int i = 0; i < 16; ++i) {
+            const uint8_t* src = sm.kq[st] + (i >> 3) * kHalf + lt * 128 + (((i & 7) ^ (lt & 7)) << 4);
+            const uint4 kv = *reinterpret_cast<const uint4*>(src), qv = *reinterpret_cast<const uint4*>(src + kC * 128);
+            k4[0] = square2(kv.x, k4[0]); q4[0] = square2(qv.x, q4[0]);
+            k4[1] = square2(kv.y, k4[1]); q4[1] = square2(qv.y, q4[1]);
+            k4[0] = square2(kv.z, k4[0]); q4[0] = square2(qv.z, q4[0]);
+            k4[1] = square2(kv.w, k4[1]); q4[1] = square2(qv.w, q4[1]);
+          }
+          float a, b;
+          unf2(fma2(k4[0], f2(1.f, 1.f), k4[1]), a, b);
+          k2 = a + b;
+          unf2(fma2(q4[0], f2(1.f, 1.f), q4[1]), a, b);
+          q2 = a + b;
+          bad |= !(k2 < INFINITY) && lt > 0;
+        }
+        if (bar_any(3, 96, bad)) {               // rare: end the chunk in front of such a token
+          if (warp == 15) {
+            int first_bad = n;
+#pragma unroll 1
+            for (int row = n - 1; row > 0; --row) {
+              const uint2 v = *reinterpret_cast<const uint2*>(sm.v[st] + row * 256 + lane * 8);
+              const uint2 k = *reinterpret_cast<const uint2*>(sm.kq[st] + (lane >> 4) * kHalf + row * 128 + (lane & 15) * 8);
+              const uint32_t z = times_zero(v.x, times_zero(v.y, times_zero(k.x, times_zero(k.y, 0))));
+              const int64_t at = (tok0 + row) * p.Hv + hv;
+              if (__any_sync(0xffffffffu, (z & 0x7fff7fffu) != 0 || !(fabsf(p.beta[at]) < INFINITY) || !(p.g[at] < INFINITY))) first_bad = row;
+            }
+            if (lane == 0) sm.cut = first_bad;
+          }
+          bar_sync(3, 96);
+          n = sm.cut;
+          if (lt >= n && lt < kC) {              // no gates behind the end: the sums stay what they are there
+            sc.gh[lt] = sc.gh[n - 1];
+            sc.gl[lt] = sc.gl[n - 1];
+          }
+          bar_sync(3, 96);
+        }
+        if (lt >= n && warp < 15) {              // rows behind the chunk's end are the next one's or another request's: zeros
+          beta = k2 = q2 = 0.f;
 #pragma unroll 2
           for (int i = 0; i < 16; ++i) {
             uint8_t* dst = sm.kq[st] + (i >> 3) * kHalf + lt * 128 + ((i & 7) << 4);
@@ -490,32 +576,22 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(const __grid_con
             *reinterpret_cast<uint4*>(dst + kC * 128) = make_uint4(0, 0, 0, 0);
             *reinterpret_cast<uint4*>(sm.v[st] + lt * 256 + i * 16) = make_uint4(0, 0, 0, 0);
           }
-        } else {
-#pragma unroll 4
-          for (int i = 0; i < 16; ++i) {
-            const uint8_t* src = sm.kq[st] + (i >> 3) * kHalf + lt * 128 + (((i & 7) ^ (lt & 7)) << 4);
-            const uint4 kv = *reinterpret_cast<const uint4*>(src), qv = *reinterpret_cast<const uint4*>(src + kC * 128);
-            k2[0] = square2(kv.x, k2[0]); q2[0] = square2(qv.x, q2[0]);
-            k2[1] = square2(kv.y, k2[1]); q2[1] = square2(qv.y, q2[1]);
-            k2[0] = square2(kv.z, k2[0]); q2[0] = square2(qv.z, q2[0]);
-            k2[1] = square2(kv.w, k2[1]); q2[1] = square2(qv.w, q2[1]);
-          }
         }
-        float ka, kb, qa, qb;
-        unf2(fma2(k2[0], f2(1.f, 1.f), k2[1]), ka, kb);
-        unf2(fma2(q2[0], f2(1.f, 1.f), q2[1]), qa, qb);
-        bar_sync(3, 64);
-        const float rk = rsqrtf(ka + kb + 1e-6f), rq = p.scale * rsqrtf(qa + qb + 1e-6f), e = ex2(sc.gh[lt] + sc.gl[lt]);
-        sc.beta[lt] = beta;
-        sc.rk[lt] = rk;
-        sc.rq[lt] = rq;
-        sc.c1[lt] = beta * e * rk;
-        sc.c2[lt] = ex2((sc.gh[kC - 1] - sc.gh[lt]) + (sc.gl[kC - 1] - sc.gl[lt])) * rk;
-        sc.c3[lt] = e * rq;
-        if (lt == kC - 1) sc.decay = e;
-        fence_proxy_async_smem();
-        mbar_arrive(&sm.full[st]);
-        bar_sync(3, 64);                         // warp 13 writes the sums of the next chunk
+        pos += n;
+        if (warp < 15) {
+          const float rk = rsqrtf(k2 + 1e-6f), rq = p.scale * rsqrtf(q2 + 1e-6f), e = ex2(sc.gh[lt] + sc.gl[lt]);
+          sc.beta[lt] = beta;
+          sc.rk[lt] = rk;
+          sc.rq[lt] = rq;
+          sc.c1[lt] = beta * e * rk;
+          sc.c2[lt] = ex2((sc.gh[kC - 1] - sc.gh[lt]) + (sc.gl[kC - 1] - sc.gl[lt])) * rk;
+          sc.c3[lt] = e * rq;
+          if (lt == kC - 1) sc.decay = e;
+          if (lt == 0) sc.n = n;
+          fence_proxy_async_smem();
+          mbar_arrive(&sm.full[st]);
+        }
+        bar_sync(3, 96);                         // the next chunk's sums and cuts are written
       }
       if (lt == 0 && failed)                     // copies in flight land before the shared memory goes away (bounded)
         for (int c = max(0, issued - 2); c < issued; ++c)
@@ -559,8 +635,10 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(const __grid_con
     wait_one(&sm.full[0], 0, 920);
     tc_fence_after_sync();
     products(0);
-    for (int c = 0; c < n_chunks; ++c) {
+    int left = L;
+    for (int c = 0; left > 0; ++c) {
       const uint32_t kq = kq_addr + (c & 1) * kStage;
+      take_chunk(sm.sc[c & 1].n, left);
       wait_one(&sm.s_ready, c, 921);
       tc_fence_after_sync();
       state_times(kX1, kq);
@@ -569,7 +647,7 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(const __grid_con
       state_times(kX2, kq + kC * 128);
       umma_commit(&sm.x2);
       // the next chunk's products of keys as early as its loads allow, but not in the way of this chunk's chain
-      bool ahead = c + 1 == n_chunks;
+      bool ahead = left == 0;
       for (int turn = 0; turn < 2; ++turn) {
         if (!ahead && (turn == 1 || mbar_try_wait(&sm.full[(c + 1) & 1], ((c + 1) >> 1) & 1))) {
           wait_one(&sm.full[(c + 1) & 1], (c + 1) >> 1, 925);

@@ -200,6 +200,42 @@ def test_gated_delta_rule_many_chunks(lens):
     torch.testing.assert_close(got.float(), want.float(), atol=1e-3, rtol=2 ** -7)
 
 
+@pytest.mark.parametrize("bad", ["v", "k", "q", "g", "beta"])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf")])
+@pytest.mark.parametrize("at", [[77], [64], [0], [70, 71, 127, 200]])
+def test_gated_delta_rule_bad_values_reach_later_tokens_only(bad, value, at):
+    """A NaN or an infinity in tokens of the first of two requests: where the scan's outputs and states are finite the chunk form's
+    are, and equal within the bounds given above; where the scan's are not, neither are they.  The other request, whose rows share
+    a tile with the bad ones, keeps its bits, and so do tokens in front of the first bad one."""
+    from vllm_kunlun_b200.ops.gemm_cuda import check_status
+    torch.manual_seed(22)
+    lens, Hk, Hv = [233, 90], 1, 2
+    T = sum(lens)
+    q, k, v = (torch.randn(T, h, 128).bfloat16() for h in (Hk, Hk, Hv))
+    g, beta = -torch.rand(T, Hv) * 0.1, torch.rand(T, Hv)
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32)
+    slots, init = torch.arange(2).int(), torch.ones(2).int()
+    states = torch.randn(2, Hv, 128, 128) * 0.1
+
+    def run(dev):
+        st = states.to(dev)
+        o = ops.gated_delta_rule(*(t.to(dev) for t in (q, k, v, g, beta)), st, cu.to(dev), slots.to(dev), init.to(dev))
+        return o.cpu().float(), st.cpu()
+
+    clean = run(DEV)
+    t = dict(q=q, k=k, v=v, g=g, beta=beta)[bad]
+    for i in at:
+        t[i].view(-1)[1 if bad in ("g", "beta") else 5] = value
+    got, want = run(DEV), run("cpu")
+    check_status()
+    assert torch.equal(got[0][:at[0]], clean[0][:at[0]])
+    assert torch.equal(got[0][lens[0]:], clean[0][lens[0]:]) and torch.equal(got[1][1], clean[1][1])
+    for a, b, tol in ((got[0], want[0], dict(atol=1e-3, rtol=2 ** -7)), (got[1], want[1], dict(atol=1e-4, rtol=1e-4))):
+        assert torch.equal(torch.isfinite(a), torch.isfinite(b))
+        ok = torch.isfinite(b)
+        torch.testing.assert_close(a[ok], b[ok], **tol)
+
+
 @pytest.mark.parametrize("lens,Hk,Hv,Dv,dtype", [([1] * 5, 2, 4, 128, torch.bfloat16), ([2, 0, 1, 3], 1, 2, 64, torch.float16),
                                                  ([1, 1, 2], 2, 2, 32, torch.float32)])
 @pytest.mark.parametrize("l2norm", [True, False])
