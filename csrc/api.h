@@ -419,7 +419,8 @@ int b200_gdn_gating(float* g, float* beta, const void* a, int64_t a_stride, cons
 int b200_gdn_recurrent(void* out, int64_t o_stride, const void* q, const void* k, int64_t qk_stride, const void* v,
                        int64_t v_stride, const float* g, const float* beta, float* states, const int* cu,
                        const int* slots, const void* has_init, int init_wide, int R, int Hk, int Hv, int Dk, int Dv, float scale,
-                       int l2norm, int dtype, int64_t T, int* status, cudaStream_t st);
+                       int l2norm, int dtype, int64_t T, const int* lens, int num_sms, int* status, cudaStream_t st);
+int b200_gdn_route(int64_t T, int R, int Hv, int num_sms, int chunkable, const int* lens, int* step);
 // Linear recurrences with a matrix state (linear_attn/recurrence.cu); kind 0 = delta rule with a decay per key channel,
 // 1 = fixed decay per head.  q, k: [T][Hk][Dk], v: [T][H][Dv] column slices of one row-strided tensor.
 typedef struct RecurrenceArgs {

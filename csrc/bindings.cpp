@@ -8,6 +8,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include <limits.h>
+
 #include <atomic>
 #include <mutex>
 #include <unordered_map>
@@ -1455,27 +1457,58 @@ void gdn_gating(at::Tensor g, at::Tensor beta, const at::Tensor& a, const at::Te
         "gdn_gating");
 }
 
+// Rows of each of R requests from the host's offsets; an empty list where they are not usable as such.
+std::vector<int> host_lengths(const c10::optional<at::Tensor>& cu, int64_t R) {
+  std::vector<int> lens;
+  if (!cu.has_value() || !cu->is_cpu() || cu->dim() != 1 || cu->size(0) < R + 1 || !cu->is_contiguous()) return lens;
+  auto fill = [&](auto* p) {
+    for (int64_t r = 0; r < R; ++r) lens.push_back((int)(p[r + 1] - p[r]));
+  };
+  if (cu->scalar_type() == at::kInt) fill(cu->data_ptr<int>());
+  else if (cu->scalar_type() == at::kLong) fill(cu->data_ptr<int64_t>());
+  return lens;
+}
+
+// (rows of a request from which the chunk kernel takes it, or 0; whether the others take the step kernel): see b200_gdn_route
+std::tuple<int64_t, bool> gdn_route(int64_t T, int64_t R, int64_t Hv, int64_t num_sms, bool chunkable, const c10::optional<at::Tensor>& cu_host) {
+  const std::vector<int> lens = host_lengths(cu_host, R);
+  int step = 0;
+  const int m = b200_gdn_route(T, (int)R, (int)Hv, (int)num_sms, chunkable, lens.empty() ? nullptr : lens.data(), &step);
+  return {m == INT_MAX ? 0 : m, step != 0};
+}
+
 void gdn_recurrent(at::Tensor out, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& g,
                    const at::Tensor& beta, at::Tensor states, const at::Tensor& cu, const at::Tensor& slots,
-                   const at::Tensor& has_init, double scale, bool l2norm) {
+                   const at::Tensor& has_init, double scale, bool l2norm, const c10::optional<at::Tensor>& cu_host) {
   // q, k [T, Hk, Dk] (same row stride), v [T, Hv, Dv], out [T, Hv, Dv], states [slots, Hv, Dv, Dk] fp32
   TORCH_CHECK(q.dim() == 3 && q.stride(2) == 1 && q.stride(1) == q.size(2) && k.stride(0) == q.stride(0) &&
               k.stride(1) == k.size(2) && v.stride(2) == 1 && v.stride(1) == v.size(2) && out.stride(1) == out.size(2));
   TORCH_CHECK(states.scalar_type() == at::kFloat && states.is_contiguous() && g.is_contiguous() && beta.is_contiguous());
   c10::cuda::CUDAGuard guard(q.device());
-  GemmState& gs = gemm_state();
-  std::lock_guard<std::mutex> lk(gs.mu);
-  if (gs.num_sms == 0) {
-    gs.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-    gs.ws = at::empty({16 << 20}, q.options().dtype(at::kFloat));
-    gs.counters = at::zeros({1 << 16}, q.options().dtype(at::kInt));
-    gs.status = at::zeros({1}, q.options().dtype(at::kInt));
+  const int num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  const std::vector<int> lens = host_lengths(cu_host, slots.size(0));
+  const int* host = lens.empty() ? nullptr : lens.data();
+  int* status = nullptr;   // of the chunk kernel, where it can serve the call
+  int step;
+  // normalised q and k only: the inverse that the chunk form needs is of a matrix whose entries the norms bound
+  const bool chunkable = q.scalar_type() == at::kBFloat16 && l2norm && q.size(2) == 128 && v.size(2) == 128;
+  if (chunkable && slots.size(0) > 0 &&
+      b200_gdn_route(q.size(0), (int)slots.size(0), (int)v.size(1), num_sms, 1, host, &step) != INT_MAX) {
+    GemmState& gs = gemm_state();
+    std::lock_guard<std::mutex> lk(gs.mu);
+    if (gs.num_sms == 0) {
+      gs.num_sms = num_sms;
+      gs.ws = at::empty({16 << 20}, q.options().dtype(at::kFloat));
+      gs.counters = at::zeros({1 << 16}, q.options().dtype(at::kInt));
+      gs.status = at::zeros({1}, q.options().dtype(at::kInt));
+    }
+    status = gs.status.data_ptr<int>();
   }
   check(b200_gdn_recurrent(out.data_ptr(), out.stride(0), q.data_ptr(), k.data_ptr(), q.stride(0), v.data_ptr(), v.stride(0),
                            g.data_ptr<float>(), beta.data_ptr<float>(), states.data_ptr<float>(), cu.data_ptr<int>(),
                            slots.data_ptr<int>(), has_init.data_ptr(), flag_width(has_init), (int)slots.size(0), (int)q.size(1),
                            (int)v.size(1), (int)q.size(2), (int)v.size(2), (float)scale, l2norm, dtype_code(q), q.size(0),
-                           gs.status.data_ptr<int>(), stream()),
+                           host, num_sms, status, stream()),
         "gdn_recurrent");
 }
 
@@ -2119,7 +2152,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("embed_stream_layernorm", &embed_stream_layernorm);
   m.def("gated_residual_layernorm", &gated_residual_layernorm);
   m.def("gdn_gating", &gdn_gating);
-  m.def("gdn_recurrent", &gdn_recurrent);
+  m.def("gdn_recurrent", &gdn_recurrent, py::arg("out"), py::arg("q"), py::arg("k"), py::arg("v"), py::arg("g"), py::arg("beta"),
+        py::arg("states"), py::arg("cu"), py::arg("slots"), py::arg("has_init"), py::arg("scale"), py::arg("l2norm"),
+        py::arg("cu_host") = py::none());
+  m.def("gdn_route", &gdn_route);
   m.def("mtp_concat_norm", &mtp_concat_norm);
   m.def("sigmoid_gate_mul", &sigmoid_gate_mul);
   m.def("lora_shrink", &lora_shrink);

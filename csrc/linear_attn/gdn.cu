@@ -221,6 +221,11 @@ constexpr int kGdnChunk = 16;
 // token and 64 tokens in chunk form 21 us (one request of 24 / 48 / 64 tokens, 32 heads: scan 18.0 / 27.5 / 35.7 us); with more
 // heads than SMs the scan's blocks share them (8 requests of 24 tokens: scan 62.6 us, chunk form 44).
 constexpr int kGdnChunkMin = 40, kGdnChunkMinMany = 16;
+// Most rows of a request for which gdn_step_kernel is launched when the lengths are known.  With SMs to spare the row counts: one
+// request, 32 heads, 2 / 4 / 8 / 16 rows: scan 11 / 12 / 14 / 18 us, step 9 / 12 / 16 / 26.  From half as many heads as SMs the
+// states' traffic does: 4 requests scan 17 / 21 / 27 / 36, step 12 / 14 / 20 / 29; 64 requests scan 117 / 146 / 197 / 283, step
+// 53 / 72 / 117 / 211.
+constexpr int kGdnStepMax = 4, kGdnStepMaxMany = 16;
 
 template <typename T, int DK>
 __global__ void __launch_bounds__(128) gdn_recurrent_kernel(
@@ -340,10 +345,11 @@ __global__ void __launch_bounds__(128) gdn_recurrent_kernel(
   for (int j = 0; j < QW; j += 4) *reinterpret_cast<float4*>(sp + j * 4) = *reinterpret_cast<const float4*>(&S[j]);
 }
 
-// The same for a token or two a request (decode, verification): bound by reading and writing the states, 128 KB a head and
+// The same for a few tokens a request (decode, verification): bound by reading and writing the states, 128 KB a head and
 // request.  A warp owns eight rows of a 128-wide state, a lane four columns of each; all eight are in flight at once, q and k
-// come straight from memory, and eight row sums are folded together (9 exchanges instead of 40).  No shared memory and no
-// barrier: 64 requests, 32 heads (268 MB) 39 us, 96 in the scan below.
+// come straight from memory, and eight row sums are folded together (9 exchanges instead of 40).  No shared memory and no barrier:
+// 64 requests, 32 heads (268 MB) 39 us, 96 in the scan above.  Some 11 us a further row there, which the exchanges and sums take: q,
+// k and v a row ahead are worth it in 32 bits only (64 requests, four rows each: 71 us, 82 without; in bf16 79, 72 without).
 __device__ __forceinline__ float sum_of_8(float (&v)[8], int lane) {   // lane l returns the sum over the warp of v[l / 4]
 #pragma unroll
   for (int h = 4; h > 0; h >>= 1) {
@@ -358,9 +364,9 @@ __device__ __forceinline__ float sum_of_8(float (&v)[8], int lane) {   // lane l
   s += __shfl_xor_sync(0xffffffff, s, 2);
   return s + __shfl_xor_sync(0xffffffff, s, 1);
 }
-template <typename T> __device__ __forceinline__ float4 ld4(const T* p) {
-  struct alignas(4 * sizeof(T)) Q { T v[4]; };
-  const Q a = *reinterpret_cast<const Q*>(p);
+template <typename T> struct alignas(4 * sizeof(T)) Four { T v[4]; };
+template <typename T> __device__ __forceinline__ Four<T> ld4(const T* p) { return *reinterpret_cast<const Four<T>*>(p); }
+template <typename T> __device__ __forceinline__ float4 to_f4(const Four<T>& a) {
   return make_float4(to_f(a.v[0]), to_f(a.v[1]), to_f(a.v[2]), to_f(a.v[3]));
 }
 
@@ -369,20 +375,31 @@ __global__ void __launch_bounds__(128) gdn_step_kernel(
     T* __restrict__ out, int64_t o_stride, const T* __restrict__ q, const T* __restrict__ k, int64_t qk_stride,
     const T* __restrict__ v, int64_t v_stride, const float* __restrict__ g, const float* __restrict__ beta,
     float* __restrict__ states /*[slots, Hv, Dv, 128]*/, const int* __restrict__ cu, const int* __restrict__ slots,
-    InitFlags has_init, int Hk, int Hv, int Dv, float scale, int l2norm) {
+    InitFlags has_init, int Hk, int Hv, int Dv, float scale, int l2norm, int limit) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int hv = blockIdx.y, r = blockIdx.z, hk = hv / (Hv / Hk), row0 = blockIdx.x * 32 + warp * 8;
   const int s = cu[r], L = cu[r + 1] - s, slot = slots[r];
-  if (L == 0 || slot < 0) return;
+  if (L == 0 || L >= limit || slot < 0) return;
   float4* sp = reinterpret_cast<float4*>(states + (((int64_t)slot * Hv + hv) * Dv + row0) * 128) + lane;
   float4 S[8];
   const bool init = has_init[r];
 #pragma unroll
   for (int i = 0; i < 8; ++i) S[i] = init ? sp[i * 32] : make_float4(0.f, 0.f, 0.f, 0.f);
+  struct Token { Four<T> k, q; T v; float g, beta; } next;   // as they are in memory: a conversion would wait for the load
+  auto fetch = [&](int t) {
+    next.k = ld4(k + t * qk_stride + hk * 128 + lane * 4);
+    next.q = ld4(q + t * qk_stride + hk * 128 + lane * 4);
+    next.v = v[t * v_stride + hv * Dv + row0 + (lane >> 2)];   // of the row whose sum this lane gets
+    next.g = g[(int64_t)t * Hv + hv];
+    next.beta = beta[(int64_t)t * Hv + hv];
+  };
+  constexpr bool kAhead = sizeof(T) == 4;
+  if (kAhead) fetch(s);
   for (int t = s; t < s + L; ++t) {
-    const float4 kk = ld4(k + t * qk_stride + hk * 128 + lane * 4), qq = ld4(q + t * qk_stride + hk * 128 + lane * 4);
-    const float gt = __expf(g[(int64_t)t * Hv + hv]), bt = beta[(int64_t)t * Hv + hv];
-    const float vt = to_f(v[t * v_stride + hv * Dv + row0 + (lane >> 2)]);   // of the row whose sum this lane gets
+    if (!kAhead) fetch(t);
+    const float4 kk = to_f4(next.k), qq = to_f4(next.q);
+    const float gt = __expf(next.g), bt = next.beta, vt = to_f(next.v);
+    if (kAhead && t + 1 < s + L) fetch(t + 1);
     float rk = 1.f, rq = scale;
     if (l2norm) {
       rk = rsqrtf(warp_sum(kk.x * kk.x + kk.y * kk.y + kk.z * kk.z + kk.w * kk.w) + 1e-6f);
@@ -513,34 +530,52 @@ extern "C" int b200_gdn_gating(float* g, float* beta, const void* a, int64_t a_s
   return cudaGetLastError() != cudaSuccess;
 }
 
+// Which kernels a call of the rule takes.  `lens`: rows of every request as the host knows them, or null.  Returns the rows of a
+// request from which gdn_chunk.cu takes it (INT_MAX: none), and in `step` whether the others go through gdn_step_kernel or the scan.
+// These are choices of speed only: the kernels go by the lengths on the device, and every length has one that serves it.
+//  - Chunks where a request is long enough.  Without `lens` the longest may have T - (R - 1) rows, each of the others one; at two
+//    rows a request or less on average all are taken for decoding or verification.
+//  - The step kernel where none of the other requests has more rows than kGdnStepMax.  63 decoding requests beside one of 2048 tokens,
+//    32 heads: 314 us with the scan for the 63, 267 with the step kernel; 64 verified requests of 2 rows 130 (an empty launch of the
+//    chunk kernel and the scan) and 53.
+extern "C" int b200_gdn_route(int64_t T_, int R, int Hv, int num_sms, int chunkable, const int* lens, int* step) {
+  const int min_len = (int64_t)R * Hv > num_sms ? b200::kGdnChunkMinMany : b200::kGdnChunkMin;
+  const int step_max = (int64_t)R * Hv > num_sms / 2 ? b200::kGdnStepMaxMany : b200::kGdnStepMax;
+  int64_t longest = T_ <= 2 * (int64_t)R ? 0 : T_ - (R - 1);
+  if (lens != nullptr) {
+    longest = 0;
+    for (int r = 0; r < R; ++r) longest = lens[r] > longest ? lens[r] : longest;
+  }
+  const bool chunk = chunkable && longest >= min_len;
+  const int chunk_min = !chunk ? INT_MAX : R == 1 ? 1 : min_len;   // a lone request needs no second launch
+  *step = lens != nullptr || longest == 0;
+  if (lens != nullptr)
+    for (int r = 0; r < R; ++r) *step &= lens[r] <= step_max || lens[r] >= chunk_min;
+  return chunk_min;
+}
+
 extern "C" int b200_gdn_recurrent(void* out, int64_t o_stride, const void* q, const void* k, int64_t qk_stride, const void* v,
                                   int64_t v_stride, const float* g, const float* beta, float* states, const int* cu,
                                   const int* slots, const void* has_init, int init_wide, int R, int Hk, int Hv, int Dk, int Dv, float scale,
-                                  int l2norm, int dtype, int64_t T_, int* status, cudaStream_t st) {
+                                  int l2norm, int dtype, int64_t T_, const int* lens, int num_sms, int* status, cudaStream_t st) {
   if (R == 0) return 0;
   if (Dv % 32 != 0 || Hv % Hk != 0) return 3;
   const b200::InitFlags flags{has_init, init_wide};
-  // Prompts go through the chunked form (4 x 2048 tokens, 32 heads: 3308 us as a scan, 221 us).  Normalised q and k only: the
-  // inverse that it needs is of a matrix whose entries the norms bound.  T_ - (R - 1) rows are the most that one request can have
-  // when each of the others has a row: decode steps go straight to the scan.
-  const int min_len = (int64_t)R * Hv > 148 ? b200::kGdnChunkMinMany : b200::kGdnChunkMin;
-  int chunk_min = INT_MAX;
-  if (dtype == b200::kBF16 && l2norm && Dk == 128 && Dv == 128 && T_ - (R - 1) >= min_len) {
-    chunk_min = R == 1 ? 1 : min_len;   // a lone request needs no second launch
+  int step, chunk_min = b200_gdn_route(T_, R, Hv, num_sms, status != nullptr, lens, &step);
+  if (chunk_min != INT_MAX) {
     const int rc = b200::gdn_chunk(out, o_stride, q, k, qk_stride, v, v_stride, g, beta, states, cu, slots, flags, T_, R, Hk,
                                    Hv, scale, chunk_min, status, st);
     if (rc > 0) return rc;
     if (rc == 0 && R == 1) return 0;
-    if (rc < 0) chunk_min = INT_MAX;
+    if (rc < 0) chunk_min = b200_gdn_route(T_, R, Hv, num_sms, 0, lens, &step);
   }
   dim3 grid(Dv / 32, Hv, R);
-  // At most two rows a request on average: the states' traffic counts, not the steps (any length is served).
   const size_t esz = dtype == b200::kF32 ? 4 : 2, vec = 4 * esz;
   auto aligned = [&](const void* x) { return reinterpret_cast<uintptr_t>(x) % vec == 0; };
-  if (Dk == 128 && T_ <= 2 * (int64_t)R && chunk_min == INT_MAX && qk_stride % 4 == 0 && aligned(q) && aligned(k)) {
+  if (step && Dk == 128 && qk_stride % 4 == 0 && aligned(q) && aligned(k)) {
     B200_DISPATCH_DTYPE(dtype, (b200::gdn_step_kernel<T><<<grid, 128, 0, st>>>(
                                    (T*)out, o_stride, (const T*)q, (const T*)k, qk_stride, (const T*)v, v_stride, g, beta,
-                                   states, cu, slots, flags, Hk, Hv, Dv, scale, l2norm)));
+                                   states, cu, slots, flags, Hk, Hv, Dv, scale, l2norm, chunk_min)));
     return cudaGetLastError() != cudaSuccess;
   }
 #define B200_GDN_LAUNCH(DK)                                                                                          \

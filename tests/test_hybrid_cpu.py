@@ -1,4 +1,5 @@
 """Qwen3-Next hybrid (gated delta net + gated attention + shared-expert MoE) on the CPU oracle path."""
+import pytest
 import torch
 
 from vllm_kunlun_b200 import LLM, SamplingParams
@@ -96,3 +97,24 @@ def test_batched_chunked_form_and_its_dispatch(monkeypatch):
     monkeypatch.setenv("B200_GDN_CHUNKED", "0")
     a = [o.token_ids for o in LLM(cfg, **kw).generate(prompts, sp)]
     assert a == b
+
+
+@pytest.mark.parametrize("lens,Hv,chunk_min,step", [
+    ([1] * 64, 32, 0, True), ([2] * 64, 32, 0, True), ([2] * 15, 32, 0, True), ([16] * 4, 32, 0, True), ([17] + [1] * 63, 32, 16, True),
+    ([2048] + [1] * 63, 32, 16, True), ([2048] * 4, 32, 40, True), ([300, 16, 1], 32, 40, True), ([300, 17, 1], 32, 40, False), ([300, 4], 32, 40, True), ([300, 5], 32, 40, False),
+    ([64], 32, 1, True), ([39], 32, 0, False), ([4], 32, 0, True), ([5], 32, 0, False), ([70] + [0] * 63, 32, 16, True)])
+def test_gated_delta_rule_route(lens, Hv, chunk_min, step):
+    """Which kernels a call takes where the host knows the lengths; 148 SMs."""
+    from vllm_kunlun_b200.ops import _ext
+    if _ext.load() is None:
+        pytest.skip("the extension is not built")
+    route = lambda cu, able=True: _ext.load().gdn_route(sum(lens), len(lens), Hv, 148, able, cu)
+    cu = torch.tensor([0] + lens).cumsum(0)
+    for host in (cu, cu.int()):
+        assert route(host) == (chunk_min, step)
+    assert route(cu, False)[0] == 0
+    # without lengths: two rows a request or less are decoding or verification
+    T, R = sum(lens), len(lens)
+    m = 16 if R * Hv > 148 else 40
+    want = (0, True) if T <= 2 * R else (1 if R == 1 else m, False) if T - R + 1 >= m else (0, False)
+    assert route(None) == want

@@ -259,6 +259,32 @@ def test_gated_delta_rule_steps(lens, Hk, Hv, Dv, dtype, l2norm):
     torch.testing.assert_close(got, want, atol=1e-5, rtol={torch.float32: 1e-4, torch.float16: 2 ** -9, torch.bfloat16: 2 ** -7}[dtype])
 
 
+@pytest.mark.parametrize("lens,Hk,Hv", [([2] * 16, 2, 16), ([1] * 9 + [150], 8, 16), ([4, 1, 3], 1, 2), ([5, 1], 1, 2), ([16, 15, 1, 7], 16, 32),
+                                        ([17, 1, 16], 16, 32), ([70] + [0] * 4, 2, 16)])
+@pytest.mark.parametrize("host", ["exact", "none", "other"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_gated_delta_rule_routes(lens, Hk, Hv, host, dtype):
+    """Verification batches, mixed steps and lengths around the limits of the step kernel: the host's lengths choose kernels, and
+    every length on the device has one that serves it, also where the host's are others (a captured step).  Bounds as above."""
+    torch.manual_seed(23)
+    T, R = sum(lens), len(lens)
+    q, k, v = (torch.randn(T, h, 128).to(dtype) for h in (Hk, Hk, Hv))
+    g, beta, states = -torch.rand(T, Hv) * 0.5, torch.rand(T, Hv), torch.randn(R + 1, Hv, 128, 128) * 0.1
+    slots, init = torch.randperm(R + 1)[:R].to(torch.int32), (torch.arange(R) % 2).to(torch.int32)
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32)
+    cu_host = dict(exact=cu.clone(), none=None, other=torch.arange(R + 1))[host]
+
+    def run(dev):
+        st = states.to(dev)
+        o = ops.gated_delta_rule(*(t.to(dev) for t in (q, k, v, g, beta)), st, cu.to(dev), slots.to(dev), init.to(dev), None, True,
+                                 cu_host if dev == DEV else None)
+        return o.cpu().float(), st.cpu()
+
+    (got, got_st), (want, want_st) = run(DEV), run("cpu")
+    torch.testing.assert_close(got_st, want_st, atol=1e-4, rtol=1e-4)
+    torch.testing.assert_close(got, want, atol=1e-3, rtol={torch.float32: 1e-4, torch.bfloat16: 2 ** -7}[dtype])
+
+
 @pytest.mark.parametrize("flags", [torch.int32, torch.bool, torch.uint8, torch.int64])
 @pytest.mark.parametrize("W", [2, 4, 9])
 def test_single_token_convolution_and_flags(flags, W):

@@ -11,8 +11,8 @@ Layout choices here (differ from the checkpoint, converted at load time):
   them per key head), so the conv input ``[q | k | v]`` is a contiguous column slice and TP shards whole heads.
 * per-request state lives in two caches indexed by the request's state slot:
   ``conv [slots, W-1, C_local]`` and ``ssm [slots, Hv_local, Dv, Dk]`` (fp32).
-* one varlen kernel serves prefill chunks and decode tokens alike (sequential scan with the state in
-  registers), so mixed batches need no prefill/decode split.
+* one varlen op serves prefill chunks and decode tokens alike (its kernels pick their requests by length on the
+  device), so mixed batches need no prefill/decode split.
 """
 from __future__ import annotations
 

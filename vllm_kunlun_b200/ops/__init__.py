@@ -658,10 +658,11 @@ GDN_CHUNK_MIN = 64      # new tokens of a request from which the chunked form is
 def gated_delta_rule(q, k, v, g, beta, states, cu_seqlens, state_indices, has_initial_state, scale=None,
                      use_qk_l2norm=True, cu_seqlens_cpu=None):
     """Varlen gated delta rule over a state cache ``[slots, Hv, Dv, Dk]`` (fp32, updated in place).
-    ``q, k [T, Hk, Dk]``, ``v [T, Hv, Dv]``, ``g, beta [T, Hv]`` fp32.  Decode steps and short requests run as a
-    scan (one dependent step per token); prompts in bf16 with 128-wide heads and normalised q and k go 64 tokens at a time
-    through the tensor cores (``csrc/linear_attn/gdn_chunk.cu``, at fp32 accuracy).  With ``B200_GDN_CHUNKED=1`` and the
-    host copy of the segment offsets, requests with at least ``GDN_CHUNK_MIN`` new tokens take the chunked form instead (the reference's
+    ``q, k [T, Hk, Dk]``, ``v [T, Hv, Dv]``, ``g, beta [T, Hv]`` fp32.  Decode and verification steps
+    have a kernel of their own, other short requests run as a scan (one dependent step per token), prompts in bf16 with 128-wide heads and
+    normalised q and k go 64 tokens at a time through the tensor cores (``csrc/linear_attn/gdn_chunk.cu``, at fp32 accuracy).
+    ``cu_seqlens_cpu``, the host copy of the segment offsets, lets a mixed step take the kernel of each kind; without it the kernels
+    are chosen from the number of rows and requests alone.  With ``B200_GDN_CHUNKED=1`` and the host copy, requests with at least ``GDN_CHUNK_MIN`` new tokens take the chunked form instead (the reference's
     prefill path, ``ops/fla/chunk.py:23-140``): batched matrix products per 64-token chunk and one state update per
     chunk; the other requests of the step keep the recurrent kernel."""
     scale = q.shape[-1] ** -0.5 if scale is None else scale
@@ -680,7 +681,8 @@ def gated_delta_rule(q, k, v, g, beta, states, cu_seqlens, state_indices, has_in
     if len(long_rows) < len(cu_seqlens) - 1:
         if q.is_cuda:
             _c().gdn_recurrent(out, q, k, v, g, beta, states, cu_seqlens.int(), slots.int(),
-                               _flags(has_initial_state), scale, use_qk_l2norm)
+                               _flags(has_initial_state), scale, use_qk_l2norm,
+                               cu_seqlens_cpu if torch.is_tensor(cu_seqlens_cpu) and not long_rows else None)
         else:
             for r in range(len(cu_seqlens) - 1):
                 s, e = int(cu_seqlens[r]), int(cu_seqlens[r + 1])
