@@ -35,13 +35,11 @@ __device__ __forceinline__ int find_seq(const int* __restrict__ cu, int R, int t
 
 // y[t, c] = act(bias[c] + sum_j w[c, j] * in[t - (W-1) + j, c]); positions before the sequence start read
 // the cached state (rows W-1+p.. of the previous inputs) or zero.
-// One thread = one 16-byte channel vector x kConvTok consecutive tokens, with a sliding window of the last W-1 input rows in
-// registers, so every input row is loaded once per thread; the loads of kConvBatch rows are in flight together.  Bound by
-// memory: 8192 tokens x 8192 channels are 268 MB (41 us); 89 us, and 140 with eight tokens
-// a thread, taps read one by one and one row in flight.
-constexpr int kConvTok = 16, kConvBatch = 8;
-
-template <typename T, int W>
+// One thread = one 16-byte channel vector x kTok consecutive tokens, with a sliding window of the last W-1 input rows in
+// registers, so every input row is loaded once per thread; the loads of kBatch rows are in flight together.  A request's first row
+// in a thread costs a chain of loads (offsets, slot, history), one request after the other, so many short requests want few
+// tokens a thread, and long ones many, for the taps and the window's first rows.
+template <typename T, int W, int kTok, int kBatch>
 __global__ void __launch_bounds__(128) conv1d_fwd_kernel(T* __restrict__ out, int64_t out_stride, const T* __restrict__ x,
                                                          int64_t x_stride, const T* __restrict__ w, const T* __restrict__ bias,
                                                          const int* __restrict__ cu, int R, const T* __restrict__ states,
@@ -49,7 +47,7 @@ __global__ void __launch_bounds__(128) conv1d_fwd_kernel(T* __restrict__ out, in
                                                          int C, int act, int64_t Ttot) {
   constexpr int V = Vec16<T>::N;
   const int c0 = (blockIdx.x * blockDim.x + threadIdx.x) * V;
-  const int64_t t0 = (int64_t)blockIdx.y * kConvTok;
+  const int64_t t0 = (int64_t)blockIdx.y * kTok;
   if (c0 >= C || t0 >= Ttot) return;
   float wv[W][V], bv[V];
   const T* wc = w + (int64_t)c0 * W;              // the V channels' taps are V * W consecutive numbers
@@ -92,13 +90,13 @@ __global__ void __launch_bounds__(128) conv1d_fwd_kernel(T* __restrict__ out, in
   };
   load_hist(t0);
 #pragma unroll 1
-  for (int i0 = 0; i0 < kConvTok; i0 += kConvBatch) {
-    Vec16<T> rows[kConvBatch];
+  for (int i0 = 0; i0 < kTok; i0 += kBatch) {
+    Vec16<T> rows[kBatch];
 #pragma unroll
-    for (int i = 0; i < kConvBatch; ++i)
+    for (int i = 0; i < kBatch; ++i)
       if (t0 + i0 + i < Ttot) rows[i] = ld_vec(x + (t0 + i0 + i) * x_stride + c0);
 #pragma unroll
-    for (int i = 0; i < kConvBatch; ++i) {
+    for (int i = 0; i < kBatch; ++i) {
       const int64_t t = t0 + i0 + i;
       if (t >= Ttot) return;
       if (t >= seq_end) {  // crossed into the next (non-empty) sequence: its history comes from its own state
@@ -472,26 +470,37 @@ int launch_conv_fwd(void* out, int64_t out_stride, const void* x, int64_t x_stri
                     int64_t T_, cudaStream_t st) {
   constexpr int V = Vec16<T>::N;
   if (C % V != 0 || (x_stride % V) != 0 || (out_stride % V) != 0) return 3;
-  dim3 g1((C / V + 127) / 128, (unsigned)((T_ + kConvTok - 1) / kConvTok)), g2((C + 255) / 256, R);
-#define B200_CONV_W(WW)                                                                                                   \
-  conv1d_fwd_kernel<T, WW><<<g1, 128, 0, st>>>((T*)out, out_stride, (const T*)x, x_stride, (const T*)w, (const T*)bias, cu, \
-                                               R, (const T*)states, slots, has_init, C, act, T_)
+  dim3 g2((C + 255) / 256, R);
+  const bool fits = T_ <= 8 * 65535;   // as blocks of eight tokens into a grid
+#define B200_CONV(WW, TOK, BATCH)                                                                                            \
+  conv1d_fwd_kernel<T, WW, TOK, BATCH><<<dim3((C / V + 127) / 128, (unsigned)((T_ + TOK - 1) / TOK)), 128, 0, st>>>(            \
+      (T*)out, out_stride, (const T*)x, x_stride, (const T*)w, (const T*)bias, cu, R, (const T*)states, slots, has_init, C, act, T_)
+  // Up to four taps: eight tokens a thread, four rows in flight (eight of 32-bit numbers, which are half as many).  us with 8 and with
+  // 16 tokens, bf16, 8192 channels, four taps: 4 x 2048 tokens 97 and 97, 64 x 1 20 and 29, 63 x 1 + 2048 42 and 52; fp32 124 and 137.
+#define B200_CONV_FEW(WW) \
+  if (fits) B200_CONV(WW, 8, (sizeof(T) == 4 ? 8 : 4)); else B200_CONV(WW, 16, 8)
+  // More: the window's first rows weigh more, so sixteen, but where requests are short and few tokens in all hide the chain.  4096
+  // channels, eight taps: 4 x 2048 tokens 125 and 95, 63 x 1 + 2048 52 and 83, 255 x 1 + 8192 165 and 132.
+#define B200_CONV_MANY(WW) \
+  if (fits && T_ < 64 * (int64_t)R && T_ * (C / V) < (2 << 20)) B200_CONV(WW, 8, 8); else B200_CONV(WW, 16, 8)
   switch (W) {
-    case 1: B200_CONV_W(1); break;
-    case 2: B200_CONV_W(2); break;
-    case 3: B200_CONV_W(3); break;
-    case 4: B200_CONV_W(4); break;
-    case 5: B200_CONV_W(5); break;
-    case 6: B200_CONV_W(6); break;
-    case 7: B200_CONV_W(7); break;
-    case 8: B200_CONV_W(8); break;
+    case 1: B200_CONV_FEW(1); break;
+    case 2: B200_CONV_FEW(2); break;
+    case 3: B200_CONV_FEW(3); break;
+    case 4: B200_CONV_FEW(4); break;
+    case 5: B200_CONV_MANY(5); break;
+    case 6: B200_CONV_MANY(6); break;
+    case 7: B200_CONV_MANY(7); break;
+    case 8: B200_CONV_MANY(8); break;
     default:
       if (T_ > 65535) return 3;
       conv1d_fwd_generic_kernel<T><<<dim3((C + 127) / 128, (unsigned)T_), 128, 0, st>>>(
           (T*)out, out_stride, (const T*)x, x_stride, (const T*)w, (const T*)bias, cu, R, (const T*)states, slots, has_init, C,
           W, act, T_);
   }
-#undef B200_CONV_W
+#undef B200_CONV_MANY
+#undef B200_CONV_FEW
+#undef B200_CONV
   if (W == 1) return cudaGetLastError() != cudaSuccess;  // no history to keep
   conv1d_state_kernel<T><<<g2, 256, 0, st>>>((T*)states, (const T*)x, x_stride, cu, slots, has_init, C, W);
   return cudaGetLastError() != cudaSuccess;

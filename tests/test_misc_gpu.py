@@ -285,6 +285,26 @@ def test_gated_delta_rule_routes(lens, Hk, Hv, host, dtype):
     torch.testing.assert_close(got, want, atol=1e-3, rtol={torch.float32: 1e-4, torch.bfloat16: 2 ** -7}[dtype])
 
 
+@pytest.mark.parametrize("W", [1, 2, 4, 5, 8])
+@pytest.mark.parametrize("lens", [[1] * 9, [7, 8, 9, 0, 1, 16], [515], [1] * 40 + [150, 3]])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_causal_conv1d_tokens_a_thread(W, lens, dtype):
+    """Short requests and long ones, around the 8 and 16 tokens that a thread takes.  Sums of at most eight products in fp32 and a
+    sigmoid to 2 units of 2^-23, rounded once to the type."""
+    torch.manual_seed(24)
+    T, R, ch = sum(lens), len(lens), 136
+    x, w, st = torch.randn(T, ch).to(dtype), torch.randn(ch, W).to(dtype), torch.randn(R + 1, W - 1, ch).to(dtype)
+    slots, init = torch.randperm(R + 1)[:R].to(torch.int32), (torch.arange(R) % 2).to(torch.int32)
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32)
+    res = []
+    for dev in (DEV, "cpu"):
+        s = st.clone().to(dev)
+        o = ops.causal_conv1d_fn(x.to(dev), w.to(dev), None, cu.to(dev), s, slots.to(dev), init.to(dev), True)
+        res.append((o.cpu().float(), s.cpu()))
+    torch.testing.assert_close(res[0][0], res[1][0], atol=1e-5, rtol=2 ** -7 if dtype == torch.bfloat16 else 1e-5)
+    assert torch.equal(res[0][1], res[1][1])
+
+
 @pytest.mark.parametrize("flags", [torch.int32, torch.bool, torch.uint8, torch.int64])
 @pytest.mark.parametrize("W", [2, 4, 9])
 def test_single_token_convolution_and_flags(flags, W):
