@@ -330,23 +330,28 @@ def test_single_token_convolution_and_flags(flags, W):
 
 
 @pytest.mark.parametrize("rows", [[300, 0, 1, 63, 64, 65], [127, 128, 129, 257]])
-@pytest.mark.parametrize("N,K,bias", [(512, 256, False), (384, 128, True), (200, 384, False)])
-def test_grouped_fp8_wide_tiles(rows, N, K, bias):
-    """128-row tiles of the fp8 grouped GEMM: empty, short and ragged groups, an odd number of weight blocks, columns off the 16-byte
-    stores.  The products of a k-block are exact in 64 bits and summed in fp32 on the GPU: K / 128 + 128 roundings of 2^-24, far
-    below the output's 2^-9, so the tolerance is that of bf16; groups without rows write nothing."""
+@pytest.mark.parametrize("N,K,bias,pitch", [(512, 256, False, 520), (384, 128, True, 384), (200, 384, False, 216), (200, 384, True, 203)])
+def test_grouped_fp8_wide_tiles(rows, N, K, bias, pitch):
+    """128-row tiles of the fp8 grouped GEMM: empty, short and ragged groups, an odd number of weight blocks, rows that 16-byte stores
+    cannot meet.  The products of a k-block are exact in 64 bits and summed in fp32 on the GPU: K / 128 + 128 roundings of 2^-24, far
+    below the output's 2^-9, so the tolerance is that of bf16.  Nothing is written behind the last group's rows (an expert-parallel
+    rank has more than its experts take), behind column N or in rows around the output."""
     from vllm_kunlun_b200.ops import _ext
+    from vllm_kunlun_b200.ops.gemm_cuda import check_status
     torch.manual_seed(13)
-    C, E, M = _ext.C(), len(rows), sum(rows)
+    C, E, used = _ext.C(), len(rows), sum(rows)
+    M = used + 150
     x = torch.randn(M, K, device=DEV).to(torch.float8_e4m3fn)
     w = torch.randn(E, N, K, device=DEV).to(torch.float8_e4m3fn)
     nb, kb = -(-N // 128), K // 128
     a_s, w_s = torch.rand(kb, (M + 3) // 4 * 4, device=DEV) + 0.1, torch.rand(E, nb, kb, device=DEV) + 0.1
     b = torch.randn(E, N, device=DEV).bfloat16() if bias else None
     lod = torch.tensor([0] + rows, device=DEV).cumsum(0).int()
-    out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    guarded = torch.full((M + 16, pitch), 12345.0, dtype=torch.bfloat16, device=DEV)
+    out = guarded[8:8 + M, :N]
     C.grouped_gemm(out, x.view(torch.uint8), w.view(torch.uint8), lod, b, a_s, w_s, 128)
-    want = torch.zeros(M, N, dtype=torch.float64, device=DEV)
+    check_status()
+    want = torch.zeros(used, N, dtype=torch.float64, device=DEV)
     for e in range(E):
         r = slice(int(lod[e]), int(lod[e + 1]))
         for i in range(kb):
@@ -354,17 +359,22 @@ def test_grouped_fp8_wide_tiles(rows, N, K, bias):
             want[r] += (x[r, c].double() @ w[e, :, c].double().T) * a_s[i, r, None].double() * w_s[e, :, i].double().repeat_interleave(128)[:N]
         if bias:
             want[r] += b[e].double()
-    torch.testing.assert_close(out.double(), want, atol=1e-2, rtol=2 ** -8)
+    torch.testing.assert_close(out[:used].double(), want, atol=1e-2, rtol=2 ** -8)
+    guarded[8:8 + used, :N] = 12345.0
+    assert bool((guarded == guarded[0, 0]).all())
 
 
 @pytest.mark.parametrize("act", [0, 1])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_grouped_fp8_with_activation(act, dtype):
-    """Activation and quantiser in the epilogue of the first expert GEMM: the bytes and scales of the kernels that it replaces."""
+    """Activation and quantiser in the epilogue of the first expert GEMM: the bytes and scales of the kernels that it replaces, and
+    none behind the last group's rows."""
     from vllm_kunlun_b200.ops import _ext
+    from vllm_kunlun_b200.ops.gemm_cuda import check_status
     torch.manual_seed(14)
     C, rows, inter, K = _ext.C(), [130, 1, 0, 64, 200], 256, 384
-    E, M = len(rows), sum(rows)
+    E, used = len(rows), sum(rows)
+    M = used + 133
     x = torch.randn(M, K, device=DEV).to(torch.float8_e4m3fn).view(torch.uint8)
     w = torch.randn(E, 2 * inter, K, device=DEV).to(torch.float8_e4m3fn).view(torch.uint8)
     a_s, w_s = torch.rand(K // 128, (M + 3) // 4 * 4, device=DEV) * 0.02, torch.rand(E, 2 * inter // 128, K // 128, device=DEV)
@@ -373,8 +383,16 @@ def test_grouped_fp8_with_activation(act, dtype):
     h = torch.empty(M, 2 * inter, dtype=dtype, device=DEV)
     C.grouped_gemm(h, x, w, lod, b, a_s, w_s, 128)
     want_q, want_s = C.act_mul_quant_fp8(h, act, lod[E:])
+    # the second call gets the first one's memory, which holds marks by then
     q, s = C.grouped_gemm_act_fp8(x, w, lod, b, a_s, w_s, act, h)
-    assert torch.equal(q, want_q) and torch.equal(s[:, :M], want_s[:, :M])
+    at = q.data_ptr(), s.data_ptr()
+    q.fill_(0xA5)
+    s.fill_(-7.0)
+    del q, s
+    q, s = C.grouped_gemm_act_fp8(x, w, lod, b, a_s, w_s, act, h)
+    check_status()
+    assert torch.equal(q[:used], want_q[:used]) and torch.equal(s[:, :used], want_s[:, :used])
+    assert (q.data_ptr(), s.data_ptr()) == at and bool((q[used:] == 0xA5).all()) and bool((s[:, used:] == -7.0).all())
 
 
 @pytest.mark.parametrize("T,k,H,mapped", [(129, 8, 256, False), (300, 4, 2048 + 128, True)])
