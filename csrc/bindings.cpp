@@ -2092,6 +2092,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_int8", &gemm_int8);
   m.def("quant_int8_token", &quant_int8_token);
   m.def("set_gemm_decode_comm", &set_gemm_decode_comm);
+  m.def("grouped_bn", &grouped_bn);
   m.def("grouped_gemm_act_fp8", &grouped_gemm_act_fp8);
   m.def("grouped_gemm", &grouped_gemm, py::arg("out"), py::arg("x"), py::arg("w"), py::arg("lod"), py::arg("bias"),
         py::arg("a_scale_t"), py::arg("w_scale"), py::arg("bn"), py::arg("act") = 0);

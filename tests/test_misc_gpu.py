@@ -395,6 +395,21 @@ def test_grouped_fp8_with_activation(act, dtype):
     assert (q.data_ptr(), s.data_ptr()) == at and bool((q[used:] == 0xA5).all()) and bool((s[:, used:] == -7.0).all())
 
 
+@pytest.mark.parametrize("T,wide", [(2, False), (64, False), (300, True)])
+def test_experts_ask_for_the_fused_epilogue_where_it_serves(T, wide, monkeypatch):
+    """A decode batch does not pay for a call that turns it down."""
+    from vllm_kunlun_b200.ops import _ext
+    torch.manual_seed(25)
+    C, E, H, inter, seen = _ext.C(), 8, 256, 128, []
+    w13, w2 = (torch.randn(E, n, m, device=DEV).to(torch.float8_e4m3fn) for n, m in ((2 * inter, H), (H, inter)))
+    s13, s2 = torch.rand(E, 2 * inter // 128, H // 128, device=DEV), torch.rand(E, H // 128, inter // 128, device=DEV)
+    inner = C.grouped_gemm_act_fp8
+    monkeypatch.setattr(C, "grouped_gemm_act_fp8", lambda *a: (seen.append(inner(*a)), seen[-1])[1])
+    w, ids = ops.moe_route(torch.randn(T, E, device=DEV), 2, "softmax", True)
+    ops.fused_moe(torch.randn(T, H, device=DEV).bfloat16(), w13, w2, w, ids, "silu", w13_scale=s13, w2_scale=s2)
+    assert len(seen) == wide and all(seen)
+
+
 @pytest.mark.parametrize("T,k,H,mapped", [(129, 8, 256, False), (300, 4, 2048 + 128, True)])
 def test_moe_permute_quant(T, k, H, mapped):
     """Rows quantised on their way to their experts: every pair's row is the quantised row of its token, pairs of other ranks' experts

@@ -64,13 +64,15 @@ def fused_moe_cuda(x, w13, w2, topk_weights, topk_ids, act="silu", b13=None, b2=
     y = torch.empty(M, H, dtype=x.dtype, device=x.device)
     if fp8:
         fuse, code = act in ("silu", "gelu_tanh") and SMALL_BATCH_FUSION[0], 0 if act == "silu" else 1
+        w13_bytes = w13.view(torch.uint8)
         # many rows an expert: activation and quantiser in the first GEMM's epilogue
-        done = C.grouped_gemm_act_fp8(q, w13.view(torch.uint8), lod, b13, st, w13_scale, code, x) if fuse else None
+        wide = fuse and C.grouped_bn(True, M, E_local) == 128
+        done = C.grouped_gemm_act_fp8(q, w13_bytes, lod, b13, st, w13_scale, code, x) if wide else None
         if done:
             q2, st2 = done
         else:
             h = torch.empty(M, w13.shape[1], dtype=x.dtype, device=x.device)
-            C.grouped_gemm(h, q, w13.view(torch.uint8), lod, b13, st, w13_scale, 0)
+            C.grouped_gemm(h, q, w13_bytes, lod, b13, st, w13_scale, 0)
             if fuse:
                 q2, st2 = C.act_mul_quant_fp8(h, code, lod[E_local:])  # activation + quantiser fused
             else:
