@@ -428,8 +428,10 @@ extern "C" int b200_qkv_split_norm_rope_cache(void* q_out, const void* qkv, cons
   auto aligned = [](const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; };
   if (D == 128 && rot_dim == 128 && neox && dtype != kF32 && qkv_stride % 8 == 0 && (q_w == nullptr) == (k_w == nullptr) &&
       aligned(qkv) && aligned(q_out) && aligned(cos_sin) && aligned(kv_cache) && aligned(q_w) && aligned(k_w)) {
-    // few tokens: a CTA per sixteen heads, so that a decode step is one turn deep
-    const dim3 grid((unsigned)T_, T_ <= 256 ? (unsigned)((Hq + 2 * Hkv + 15) / 16) : 1u);
+    // Few tokens: a CTA per sixteen heads, so that a decode step is one turn deep; then one per token, which reads its cosines
+    // once.  us with the first and the second, 32 + 16 heads: 1 token 2.4 and 2.8, 128 3.3 and 4.6, 384 4.7 and 5.1, 512 6.0 and
+    // 5.3, 2048 17.3 and 11.8; 64 + 16 heads 384 tokens 6.7 and 6.8, 512 8.3 and 7.0.
+    const dim3 grid((unsigned)T_, T_ <= 384 ? (unsigned)((Hq + 2 * Hkv + 15) / 16) : 1u);
     if (dtype == kBF16)
       launch_pdl(qkv_split_norm_rope_cache_128_kernel<__nv_bfloat16>, grid, dim3(256), 0, st, (__nv_bfloat16*)q_out,
                  (const __nv_bfloat16*)qkv, positions, cos_sin, (const __nv_bfloat16*)q_w, (const __nv_bfloat16*)k_w, eps, Hq, Hkv,
