@@ -14,8 +14,12 @@
 // What bounds it: per tile the tensor core needs 1024 cycles (2 x 128^3 products), the special-function units 1024 (128 x
 // 128 exponentials at 16 a cycle); with two streams both are shared by two tiles.  P goes through TMEM because a
 // product with both operands in shared memory reads 64 KB for 512 cycles, all that shared memory delivers.
-// 384 threads: warp 0 TMA producer, warp 1 MMA issuer, warps 4-7 / 8-11 softmax and epilogue of stream 0 / 1.  CTAs take
-// work items longest first, in snake order.  TMA loads carry no cluster multicast.  Every wait is bounded; on time-out
+// 384 threads: warp 0 TMA producer, warp 1 MMA issuer, warps 4-7 / 8-11 softmax and epilogue of stream 0 / 1.  The grid has a CTA per
+// work item, in descending order of row blocks, and a CTA that is done cancels the launch of the next pending one and takes its
+// item (cluster launch control): items of one call differ a hundredfold where prompts or their contexts do, which a fixed
+// distribution cannot balance.  us with items dealt out in turn, and now: 37 requests of 16 heads, one of 4096 tokens, the others
+// 16: 1031 and 130 (425 with one tile a CTA); 512 tokens each, one behind 16000: 919 and 297 (386); 11 ragged prompts 40 and 31; 4 x
+// 2048 tokens 173 and 170.  TMA loads carry no cluster multicast.  Every wait is bounded; on time-out
 // the status word is set and the CTA unwinds.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -64,7 +68,8 @@ struct Params {
   int units;                // head pairs (by_heads) or heads
   int by_heads;             // streams are two heads over the same rows, otherwise two row tiles of one head
   int single;               // one stream only: as many CTAs as there are tiles
-  int row_blocks, items, B;
+  int row_blocks, B;
+  int take;                // CTAs may be pending: whoever is done takes their items
   int64_t num_blocks;
   float scale_log2;
 };
@@ -157,13 +162,9 @@ struct Item {
   int n_max;
 };
 
-// The `round`-th item of this CTA, or false when there is none left.  Items are ordered by descending row block, so by
-// descending number of key tiles for prompts of one length; odd rounds run through the CTAs backwards.
+// Item `idx` of the call.  Items are ordered by descending row block, so by descending number of key tiles for prompts of one length.
 template <bool kMla>
-__device__ __forceinline__ bool get_item(const Params& p, int round, Item& it) {
-  const int G = gridDim.x, c = (round & 1) ? G - 1 - (int)blockIdx.x : (int)blockIdx.x;
-  const int idx = round * G + c;
-  if (idx >= p.items) return false;
+__device__ __forceinline__ void get_item(const Params& p, int idx, Item& it) {
   const int per = p.B * p.units, rb = p.row_blocks - 1 - idx / per, rem = idx % per;
   it.req = rem / p.units;
   const int u = rem % p.units;
@@ -189,7 +190,26 @@ __device__ __forceinline__ bool get_item(const Params& p, int round, Item& it) {
     it.n[s] = max(0, (kv_end - it.kv_begin + kTile - 1) / kTile);
     it.n_max = max(it.n_max, it.n[s]);
   }
-  return true;
+}
+
+// Asks for the index of a CTA of this grid that has not been started, which then never will be: 16 bytes at `dst`, complete_tx on `bar`.
+__device__ __forceinline__ void ask_for_cta(uint32_t dst, uint64_t* bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(dst),
+               "r"(smem_u32(bar)) : "memory");
+}
+// The answer: a CTA's index, or -1 when all have been started or taken (then no further question may be asked).
+__device__ __forceinline__ int taken_cta(uint32_t src) {
+  uint32_t ok, x = 0;
+  asm volatile(
+      "{\n\t.reg .b128 r;\n\t.reg .b64 lo, hi;\n\t.reg .pred p;\n\t"
+      "ld.shared.v2.b64 {lo, hi}, [%2];\n\t"
+      "mov.b128 r, {lo, hi};\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "mov.u32 %1, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, r;\n\t}"
+      : "=r"(ok), "=r"(x) : "r"(src) : "memory");
+  return ok ? (int)x : -1;
 }
 
 template <typename T, bool kMla>
@@ -213,7 +233,11 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint64_t* s_full = bars + 16;         // [2 streams]
   uint64_t* p_ready = bars + 18;        // [2 streams][2 halves] one arrival per softmax warp
   uint64_t* o_final = bars + 22;        // [2 streams] one phase per item with work for the stream
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
+  // answers about the next item: question k uses slot k & 1
+  uint64_t* next_full = bars + 24;      // [2]
+  uint64_t* next_empty = bars + 26;     // [2] read by the MMA thread and the eight softmax warps
+  const uint32_t next_at = smem_u32(bars + 28);   // [2] x 16 bytes
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 32);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -228,6 +252,8 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       mbar_init(&s_full[s], 1);
       mbar_init(&o_final[s], 1);
       for (int h = 0; h < 2; ++h) mbar_init(&p_ready[s * 2 + h], 4);
+      mbar_init(&next_full[s], 1);
+      mbar_init(&next_empty[s], 9);
     }
     mbar_fence_init();
     prefetch_tmap(&tmQ);
@@ -245,81 +271,112 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const uint32_t tmem_base = *tmem_slot;
   griddep_wait();   // q, the lengths and this step's cache rows come from the preceding kernels
   Item it;
+  // MMA thread, softmax warps: answer k.  -1: there is no further item, or a wait gave up (then `ok` is false as well).
+  auto next_item = [&](int k, bool whole_warp, bool& ok) {
+    if (!p.take) return -1;
+    ok = wait_or_abort(&next_full[k & 1], (k >> 1) & 1, ab, 829);
+    if (whole_warp) ok = !__any_sync(0xffffffffu, !ok);
+    if (!ok) return -1;
+    const int idx = taken_cta(next_at + 16 * (k & 1));
+    fence_proxy_async_smem();           // read before the next answer is written here
+    if (whole_warp) __syncwarp();
+    if (!whole_warp || lane == 0) mbar_arrive(&next_empty[k & 1]);
+    return idx;
+  };
 
   if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (elect_one()) {
-      int kc = 0, vc = 0, qc = 0;    // K tiles, V pages and items issued so far
+      int kc = 0, vc = 0, qc = 0, asked = 0;    // K tiles, V pages and items issued, questions asked so far
       bool ok = true;
-      for (int round = 0; ok && get_item<kMla>(p, round, it); ++round) {
-        if (it.n_max == 0) continue;
+      // asked when the item's last loads are due: late enough that a CTA does not hold an item it cannot start, early enough that the
+      // answer is there before the last tiles have been worked on
+      auto ask = [&]() {
+        const int b = asked & 1;
+        if (asked >= 2 && !wait_or_abort(&next_empty[b], ((asked >> 1) - 1) & 1, ab, 830)) return false;
+        mbar_expect_tx(&next_full[b], 16);
+        ask_for_cta(next_at + 16 * b, &next_full[b]);
+        ++asked;
+        return true;
+      };
+      for (int idx = blockIdx.x; ok && idx >= 0;) {
+        get_item<kMla>(p, idx, it);
         const int n_max = it.n_max;
-        if (qc > 0 && !wait_or_abort(q_empty, (qc - 1) & 1, ab, 820)) { ok = false; break; }
-        mbar_expect_tx(q_full, kKBytes * ((it.n[0] > 0) + (it.n[1] > 0)));
+        if (n_max > 0) {
+          if (qc > 0 && !wait_or_abort(q_empty, (qc - 1) & 1, ab, 820)) { ok = false; break; }
+          mbar_expect_tx(q_full, kKBytes * ((it.n[0] > 0) + (it.n[1] > 0)));
 #pragma unroll
-        for (int s = 0; s < 2; ++s)
-          if (it.n[s] > 0) {
+          for (int s = 0; s < 2; ++s)
+            if (it.n[s] > 0) {
 #pragma unroll
-            for (int h = 0; h < kQBlocks; ++h)
-              tma_load_2d(sQ + s * kKBytes + h * kBlockBytes, &tmQ, q_full, it.head[s] * (kQBlocks * 64) + h * 64,
-                          it.qs + it.row0[s]);
-          }
-        ++qc;
-        const int* bt = kMla ? nullptr : p.block_tables + (int64_t)it.req * p.max_blocks;
-        const int kvh = it.head[0] / (p.Hq / p.Hkv), kv_row0 = kMla ? p.kv_starts[it.req] : 0;
-        const int key_end = min(it.seq_len, it.kv_begin + n_max * kTile);
-        // cache row of a key's page (paged form): masked keys read any initialised page
-        auto page_row = [&](int key) -> int64_t {
-          const int bi = key / p.block_size;
-          int64_t blk = (key < key_end && bi < p.max_blocks) ? bt[bi] : 0;
-          if (blk < 0 || blk >= p.num_blocks) blk = 0;
-          return ((blk * 2) * p.Hkv + kvh) * p.block_size + (key % p.block_size);
-        };
-        for (int j = 0; ok && j <= n_max; ++j) {      // K(0), K(1), V(0), K(2), V(1), ...
-          if (j < n_max) {
-            const int st = kc % kKStages, use = kc / kKStages;
-            if (use > 0 && !wait_or_abort(&k_empty[st], (use - 1) & 1, ab, 821)) { ok = false; break; }
-            mbar_expect_tx(&k_full[st], kKBytes);
+              for (int h = 0; h < kQBlocks; ++h)
+                tma_load_2d(sQ + s * kKBytes + h * kBlockBytes, &tmQ, q_full, it.head[s] * (kQBlocks * 64) + h * 64,
+                            it.qs + it.row0[s]);
+            }
+          ++qc;
+          const int* bt = kMla ? nullptr : p.block_tables + (int64_t)it.req * p.max_blocks;
+          const int kvh = it.head[0] / (p.Hq / p.Hkv), kv_row0 = kMla ? p.kv_starts[it.req] : 0;
+          const int key_end = min(it.seq_len, it.kv_begin + n_max * kTile);
+          // cache row of a key's page (paged form): masked keys read any initialised page
+          auto page_row = [&](int key) -> int64_t {
+            const int bi = key / p.block_size;
+            int64_t blk = (key < key_end && bi < p.max_blocks) ? bt[bi] : 0;
+            if (blk < 0 || blk >= p.num_blocks) blk = 0;
+            return ((blk * 2) * p.Hkv + kvh) * p.block_size + (key % p.block_size);
+          };
+          for (int j = 0; ok && j <= n_max; ++j) {      // K(0), K(1), V(0), K(2), V(1), ...
+            if (j == n_max - 1 && p.take && !ask()) { ok = false; break; }
+            if (j < n_max) {
+              const int st = kc % kKStages, use = kc / kKStages;
+              if (use > 0 && !wait_or_abort(&k_empty[st], (use - 1) & 1, ab, 821)) { ok = false; break; }
+              mbar_expect_tx(&k_full[st], kKBytes);
 #pragma unroll
-            for (int pg = 0; pg < kTile / kPage; ++pg) {
-              const int key = it.kv_begin + j * kTile + pg * kPage;
-              uint8_t* dst = sK + st * kKBytes + pg * (kPage * 128);
-              if constexpr (kMla) {
-                // rows past the request's keys belong to the next request or lie outside the tensor (zero fill): masked
+              for (int pg = 0; pg < kTile / kPage; ++pg) {
+                const int key = it.kv_begin + j * kTile + pg * kPage;
+                uint8_t* dst = sK + st * kKBytes + pg * (kPage * 128);
+                if constexpr (kMla) {
+                  // rows past the request's keys belong to the next request or lie outside the tensor (zero fill): masked
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
-                  tma_load_2d(dst + h * kBlockBytes, &tmKV, &k_full[st], it.head[0] * 256 + h * 64, kv_row0 + key);
-                tma_load_2d(dst + 2 * kBlockBytes, &tmKpe, &k_full[st], 0, kv_row0 + key);
-              } else {
-                const int64_t row = page_row(key);
+                  for (int h = 0; h < 2; ++h)
+                    tma_load_2d(dst + h * kBlockBytes, &tmKV, &k_full[st], it.head[0] * 256 + h * 64, kv_row0 + key);
+                  tma_load_2d(dst + 2 * kBlockBytes, &tmKpe, &k_full[st], 0, kv_row0 + key);
+                } else {
+                  const int64_t row = page_row(key);
 #pragma unroll
-                for (int h = 0; h < 2; ++h) tma_load_2d(dst + h * kBlockBytes, &tmKV, &k_full[st], h * 64, (int)row);
+                  for (int h = 0; h < 2; ++h) tma_load_2d(dst + h * kBlockBytes, &tmKV, &k_full[st], h * 64, (int)row);
+                }
+              }
+              ++kc;
+            }
+            if (j >= 1) {
+#pragma unroll
+              for (int pg = 0; pg < kTile / kPage; ++pg) {
+                const int st = vc % kVStages, use = vc / kVStages;
+                if (use > 0 && !wait_or_abort(&v_empty[st], (use - 1) & 1, ab, 822)) { ok = false; break; }
+                mbar_expect_tx(&v_full[st], kVBytes);
+                const int key = it.kv_begin + (j - 1) * kTile + pg * kPage;
+                uint8_t* dst = sV + st * kVBytes;
+                if constexpr (kMla) {
+#pragma unroll
+                  for (int h = 0; h < 2; ++h)
+                    tma_load_2d(dst + h * (kVBytes / 2), &tmKV, &v_full[st], it.head[0] * 256 + 128 + h * 64, kv_row0 + key);
+                } else {
+                  const int64_t row = page_row(key) + (int64_t)p.Hkv * p.block_size;
+#pragma unroll
+                  for (int h = 0; h < 2; ++h) tma_load_2d(dst + h * (kVBytes / 2), &tmKV, &v_full[st], h * 64, (int)row);
+                }
+                ++vc;
               }
             }
-            ++kc;
           }
-          if (j >= 1) {
-#pragma unroll
-            for (int pg = 0; pg < kTile / kPage; ++pg) {
-              const int st = vc % kVStages, use = vc / kVStages;
-              if (use > 0 && !wait_or_abort(&v_empty[st], (use - 1) & 1, ab, 822)) { ok = false; break; }
-              mbar_expect_tx(&v_full[st], kVBytes);
-              const int key = it.kv_begin + (j - 1) * kTile + pg * kPage;
-              uint8_t* dst = sV + st * kVBytes;
-              if constexpr (kMla) {
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-                  tma_load_2d(dst + h * (kVBytes / 2), &tmKV, &v_full[st], it.head[0] * 256 + 128 + h * 64, kv_row0 + key);
-              } else {
-                const int64_t row = page_row(key) + (int64_t)p.Hkv * p.block_size;
-#pragma unroll
-                for (int h = 0; h < 2; ++h) tma_load_2d(dst + h * (kVBytes / 2), &tmKV, &v_full[st], h * 64, (int)row);
-              }
-              ++vc;
-            }
-          }
+        } else if (p.take) {
+          ok = ask();
         }
+        if (!p.take) break;
+        if (!ok || !wait_or_abort(&next_full[(asked - 1) & 1], ((asked - 1) >> 1) & 1, ab, 829)) { ok = false; break; }
+        idx = taken_cta(next_at + 16 * ((asked - 1) & 1));
+        fence_proxy_async_smem();
       }
       if (!ok) {   // let the copies in flight land before the CTA's shared memory goes away (bounded)
         auto drain = [](uint64_t* bar, uint32_t parity) {
@@ -329,6 +386,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (qc > 0) drain(q_full, (qc - 1) & 1);
         for (int i = max(0, kc - kKStages); i < kc; ++i) drain(&k_full[i % kKStages], (i / kKStages) & 1);
         for (int i = max(0, vc - kVStages); i < vc; ++i) drain(&v_full[i % kVStages], (i / kVStages) & 1);
+        if (asked > 0) drain(&next_full[(asked - 1) & 1], ((asked - 1) >> 1) & 1);
       }
     }
   } else if (warp == 1) {
@@ -339,7 +397,8 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       const uint32_t idesc_o = umma_idesc(kTile, kD, fmt, fmt, 0, 1);      // A = P (TMEM), B = V tile (MN-major)
       int kc = 0, vc = 0, qc = 0, tc[2] = {0, 0};   // consumed so far; tc: tiles of each stream whose P has been awaited
       bool ok = true;
-      for (int round = 0; ok && get_item<kMla>(p, round, it); ++round) {
+      for (int idx = blockIdx.x, round = 0; idx >= 0; idx = ok ? next_item(round++, false, ok) : -1) {
+        get_item<kMla>(p, idx, it);
         if (it.n_max == 0) continue;
         const int n_max = it.n_max;
         // S of tile j of the item; the last reader of a K stage (of Q) gives it back
@@ -407,7 +466,9 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const float sc = p.scale_log2;
     int tc = 0, oc = 0;    // tiles and items of this stream so far
     bool fail = false;
-    for (int round = 0; !fail && get_item<kMla>(p, round, it); ++round) {
+    bool ok = true;
+    for (int idx = blockIdx.x, round = 0; idx >= 0; idx = next_item(round++, true, ok)) {
+      get_item<kMla>(p, idx, it);
       const int n = s ? it.n[1] : it.n[0];
       if (n == 0) continue;
       const int head = s ? it.head[1] : it.head[0], row0 = s ? it.row0[1] : it.row0[0], rows = s ? it.rows[1] : it.rows[0];
@@ -541,8 +602,8 @@ static int launch(Params& p, const CUtensorMap& tmQ, const CUtensorMap& tmKV, co
   p.row_blocks = (max_query_len + step - 1) / step;
   const int64_t items = (int64_t)p.B * p.units * p.row_blocks;
   if (items > (1 << 30)) return 3;
-  p.items = (int)items;
-  return (int)launch_pdl(kern, dim3((unsigned)(items < num_sms ? items : num_sms)), dim3(kThreads), Cfg<kMla>::kSmem, st, tmQ,
+  p.take = items > num_sms;
+  return (int)launch_pdl(kern, dim3((unsigned)items), dim3(kThreads), Cfg<kMla>::kSmem, st, tmQ,
                          tmKV, tmKpe, p);
 }
 

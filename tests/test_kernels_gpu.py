@@ -535,6 +535,74 @@ def test_prefill_attention_pairs(Hq, Hkv, window):
     _close(out, ref, 2e-2, 2e-2, f"prefill pairs window={window}")
 
 
+@pytest.mark.parametrize("lens,ctx,Hq,Hkv,dtype", [([16] * 36 + [1300], [0] * 37, 16, 2, torch.bfloat16),
+                                                   ([150] * 37, [0] * 36 + [2000], 16, 8, torch.float16), ([40] * 90, [30] * 90, 5, 5, torch.bfloat16),
+                                                   ([1, 700, 3], [0, 0, 900], 64, 8, torch.bfloat16)])
+def test_prefill_attention_uneven_batches(lens, ctx, Hq, Hkv, dtype):
+    """Many more work items than CTAs, most of them without work or of a single tile beside long ones: CTAs take items from one
+    another.  Bounds as above."""
+    from vllm_kunlun_b200.ops.attention_cuda import paged_attention_cuda
+    from vllm_kunlun_b200.ops.gemm_cuda import check_status
+    seq_lens = [a + b for a, b in zip(lens, ctx)]
+    cache, bt = _make_paged(len(lens), seq_lens, Hkv, 128, 64, dtype=dtype, seed=6)
+    qsl = torch.tensor([0] + lens).cumsum(0).to(torch.int32)
+    q = torch.randn(int(qsl[-1]), Hq, 128, generator=torch.Generator().manual_seed(10)).to(dtype)
+    sl = torch.tensor(seq_lens, dtype=torch.int32)
+    ref = ra.paged_attention(q, cache, bt, sl, qsl, 128 ** -0.5, None)
+    dev = [t.to(DEV) for t in (q, cache, bt, sl, qsl)]
+    for _ in range(3):
+        out = torch.full(q.shape, float("nan"), device=DEV, dtype=dtype)
+        paged_attention_cuda(out, *dev, 128 ** -0.5, max(lens), max(seq_lens), None)
+        _close(out, ref, 2e-2, 2e-2, "prefill uneven")
+    check_status()
+
+
+@pytest.mark.parametrize("causal", [True, False])
+def test_mla_prefill_uneven_batches(causal):
+    """The same for the latent form, with requests that have no key."""
+    from vllm_kunlun_b200.ops.gemm_cuda import check_status
+    torch.manual_seed(11)
+    N, lens = 4, [16] * 70 + [700, 3, 257, 1]
+    kv_lens = list(lens) if causal else [0 if i % 5 == 0 else 1 + 37 * i % 400 for i in range(len(lens))]
+    T, rows = sum(lens), sum(kv_lens)
+    q, kv, k_pe = torch.randn(T, N, 192).bfloat16(), torch.randn(rows, N * 256).bfloat16(), torch.randn(rows, 64).bfloat16()
+    qsl, starts = (torch.tensor([0] + v).cumsum(0).to(torch.int32) for v in (lens, kv_lens))
+    args = [q, kv, k_pe, starts[:-1].contiguous(), torch.tensor(kv_lens, dtype=torch.int32), qsl]
+    want, want_lse = ops.mla_prefill_attention(*args, causal, 192 ** -0.5, max(lens))
+    got, got_lse = ops.mla_prefill_attention(*(t.to(DEV) for t in args), causal, 192 ** -0.5, max(lens))
+    check_status()
+    _close(got, want, 2e-2, 2e-2, "mla prefill uneven")
+    torch.testing.assert_close(got_lse.cpu(), want_lse, atol=2e-2, rtol=2e-3)
+
+
+def test_prefill_attention_spreads_uneven_batches():
+    """37 requests of 16 heads are twice as many work items a row block as there are SMs, so a fixed distribution would give all of the one
+    long prompt's items to the same few CTAs (1031 us instead of 102 with 36); taken as CTAs become free, both batches take as long."""
+    from vllm_kunlun_b200.ops.attention_cuda import paged_attention_cuda
+    times = []
+    for short in (35, 36):
+        lens = [16] * short + [4096]
+        need = [-(-n // 64) for n in lens]
+        bt = torch.zeros(len(lens), 64, dtype=torch.int32)
+        order = torch.arange(sum(need), dtype=torch.int32)
+        for i, n in enumerate(need):
+            bt[i, :n] = order[sum(need[:i]):sum(need[:i + 1])]
+        cache = torch.randn(sum(need), 2, 2, 64, 128, device=DEV).bfloat16()
+        qsl, sl = torch.tensor([0] + lens).cumsum(0).int().to(DEV), torch.tensor(lens).int().to(DEV)
+        q = torch.randn(sum(lens), 16, 128, device=DEV).bfloat16()
+        out, bt = torch.empty_like(q), bt.to(DEV)
+        best = 1e9
+        for _ in range(8):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            paged_attention_cuda(out, q, cache, bt, sl, qsl, 128 ** -0.5, 4096, 4096, None)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        times.append(best)
+    assert times[1] < 2 * times[0], times
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("T,N,K,group,splits", [(1, 256, 512, 128, 0), (16, 300, 1024, 64, 0), (16, 4096, 4096, 128, 0),
                                                 (32, 1024, 2048, 128, 0), (5, 384, 4096, 128, 4), (16, 128, 4096, 4096, 8),
