@@ -12,7 +12,7 @@
 // the epilogue itself, a k-block took as long as that load (1300 cycles).
 // Measured, us (before: weights on the lanes, four epilogue warps, 128 columns a tile, activation and quantiser in a kernel
 // of their own): 4096 x 4096 x 6144 dense with the quantiser in front 148 (354); experts of 4096 tokens, 8 of 128, 2048 -> 2 x 768
-// -> 2048, with routing and permutation 393 (1031).
+// -> 2048, with routing and permutation 430 (1031).
 //
 // Fused form: the two blocks are 128 gate and the 128 up rows of the same columns; the epilogue rounds both to the model's
 // type, applies the activation and writes e4m3 with 1 x 128 scales, as act_mul_quant_fp8_kernel (moe.cu) would.

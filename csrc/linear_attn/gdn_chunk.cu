@@ -9,14 +9,15 @@
 // One CTA walks through one (request, value head); all products have the 128 rows dv as lanes.  The norms of q and k, the
 // gates and beta are applied to fp32 columns, so q and k enter the tensor core as they are in memory; every fp32 operand
 // (S, R, T, U, P) is cut into three bf16 pieces that add up to all its 24 bits, and of a product of two such
-// operands the six pairs above 2^-24 are summed: the results are those of fp32 arithmetic.  Sums of gates are kept as
+// operands six pairs are summed.  Pieces are cut and not rounded, so the pairs left out are below 2^-22 of the leading one; against 64
+// bits states are off by 1.3e-7, the scan's by 1.3e-7 to 1.4e-6.  Sums of gates are kept as
 // pairs of floats (from doubles), because a difference of two sums is what is raised to a power.
 //
 // Warps 0-3: A, T and P of the chunk ahead; warps 4-11: the chain S -> R -> U -> S, a thread = one row x half of the
 // columns, S in registers; warp 12: MMA issue; warps 13 to 15: loads, norms and gates, up to two chunks ahead.  What bounds it is that chain: three dependent products
 // (24, 24 and 12 MMA steps) with a pass through registers between them, 64 tokens a turn; the outputs and the
 // next chunk's T are computed beside it.  6 us a chunk and CTA, of which 2.9 are products (4 x 2048 tokens, 32 heads:
-// 217 us, 3308 us as a scan; 1 x 4096 tokens, 16 heads: 393 us, 1910 us as a scan).  Waits and loops are kept small (70 KB of
+// 214 us, 3308 us as a scan; 1 x 4096 tokens, 16 heads: 392 us, 1910 us as a scan).  Waits and loops are kept small (70 KB of
 // code in all): unrolled throughout, the roles evicted one another's instructions and a chunk took 13 us.  Every wait is bounded; a CTA that gives up sets the status word and runs out.
 // Zeros hide later keys, and zero times a NaN or an infinity is not zero: a chunk ends in front of a token with such a value in k,
 // v, its gate or beta, which is the first token of the next one.  So it reaches its own and later tokens only, as in the scan
